@@ -410,14 +410,17 @@ __device__ __forceinline__ void blockSumDoubles(double (&vals)[N], double* scrat
 // (jgs2-shader.ts:3097-3111): vol (a |g|^2 I + c1 u u^T + lambda w w^T) with
 // u = F g and w = cof(F) g, the stable Neo-Hookean tangent applied to the
 // rank-one direction e_i g^T.
-__device__ __forceinline__ void addIncidentBlock(S3& hess, const TetRec& r, const M3& F, const PiolaTerms& pt,
-                                                 float3 g) {
+__device__ __forceinline__ S3 incidentBlock(const TetRec& r, const M3& F, const PiolaTerms& pt, float3 g) {
   const float3 u1 = mv(F, g), w1 = mv(pt.cof, g);
   S3 blk = szero();
   saddDiag(blk, pt.a * dot3(g, g));
   saddOuter(blk, pt.c1, u1);
   saddOuter(blk, r.lambda, w1);
-  saddScaled(hess, r.vol, blk);
+  return blk;
+}
+__device__ __forceinline__ void addIncidentBlock(S3& hess, const TetRec& r, const M3& F, const PiolaTerms& pt,
+                                                 float3 g) {
+  saddScaled(hess, r.vol, incidentBlock(r, F, pt, g));
 }
 
 __device__ __forceinline__ void storeIncident(float4* __restrict__ inc, uint32_t v, float3 g, const S3& h) {
@@ -426,17 +429,23 @@ __device__ __forceinline__ void storeIncident(float4* __restrict__ inc, uint32_t
   inc[3ull * v + 2] = make_float4(h.yz, 0.0f, 0.0f, 0.0f);
 }
 
-// Vertex frame and incident system of a free vertex at pose x in one pass
-// over its incident tets: the frame is the polar of the volume-weighted
-// average F (vertexPolarRotation, jgs2-shader.ts:2959-2989), the system the
-// incident material gradient sum vol P(F) g and Hessian blocks, plus the
-// cloth membrane and bending terms of the vertex's incident elements.
-__device__ __forceinline__ void frameAndIncident(const Buffers& b, const DevParams& p, const float4* __restrict__ x,
-                                                 uint32_t v, const uint4& info, float eps) {
-  M3 avg = mzero();
-  float total = 0.0f;
-  Comp3 grad = czero();  // compensated gradient gather
-  S3 hess = szero();
+// Sums over a vertex's incident tets at one pose: the compensated material
+// gradient sum vol P(F) g, the Hessian blocks, the volume-weighted F and the
+// volume.
+struct IncidentSums {
+  Comp3 grad;
+  S3 hess;
+  M3 avg;
+  float total;
+};
+__device__ __forceinline__ IncidentSums incidentZero() { return {czero(), szero(), mzero(), 0.0f}; }
+
+// One thread per vertex: the tets in adjacency order, the next tet's record
+// requested before the current one's arithmetic so its latency overlaps the
+// work.
+template <bool kHessian>
+__device__ __forceinline__ void incidentSums(const Buffers& b, const float4* __restrict__ x, const uint4& info,
+                                             IncidentSums& o) {
 #if JGS2_CONV_LOOKAHEAD
   uint32_t nextEntry = info.y ? __ldg(&b.adjacency[info.x]) : 0u;
   TetRec nextRec;
@@ -461,17 +470,123 @@ __device__ __forceinline__ void frameAndIncident(const Buffers& b, const DevPara
     const M3 F = deformationAt(r, x);
     const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
     const float3 g = shapeGradient(r, entry & 3u);
-    cadd(grad, r.vol * mv(piola(F, pt), g));
-    addIncidentBlock(hess, r, F, pt, g);
-    avg = avg + r.vol * F;
-    total += r.vol;
+    cadd(o.grad, r.vol * mv(piola(F, pt), g));
+    if (kHessian) addIncidentBlock(o.hess, r, F, pt, g);
+    o.avg = o.avg + r.vol * F;
+    o.total += r.vol;
   }
+}
+
+// Eight lanes per vertex, for scenes too small to hide a thread's chain of 24
+// dependent tet gathers behind other warps: each lane evaluates one tet of a
+// round into its row of `rows`, then the lanes add the rows in adjacency
+// order, a few of the 19 sums each.  Every sum takes the same operands in the
+// same order and with the same fused multiply-adds as incidentSums, so both
+// give the same bits.  The sums go to `out` (kIncidentSum floats), from which
+// one thread per vertex carries on, so that the polar iterations fill a warp
+// instead of one lane of every group.
+constexpr int kIncidentLanes = 8;
+constexpr int kIncidentRow = 20;  // gradient 3, Hessian 6, F 9, 1, volume
+constexpr int kIncidentGroup = kIncidentLanes * kIncidentRow + 8;  // floats per group; groups of a warp on different banks
+constexpr int kIncidentSum = 23;  // 19 sums, 3 gradient compensations; odd, so vertices lie on different banks
+constexpr int kWideBlock = kConvChunk * kIncidentLanes;  // a reduction entry's vertices
+static_assert(kConvChunk == 32, "an entry's vertices are one warp");
+struct IncidentShared {
+  float4 rows4[kConvChunk * kIncidentGroup / 4];
+  float sums[kConvChunk][kIncidentSum];
+};
+template <bool kHessian>
+__device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4* __restrict__ x, const uint4& info,
+                                                  float* rows, uint32_t lane, unsigned mask, float* out) {
+  float s[3] = {0.0f, 0.0f, 0.0f}, c = 0.0f;
+  for (uint32_t a0 = 0; a0 < info.y; a0 += kIncidentLanes) {
+    const uint32_t n = min(info.y - a0, static_cast<uint32_t>(kIncidentLanes));
+    if (lane < n) {
+      const uint32_t entry = __ldg(&b.adjacency[info.x + a0 + lane]);
+      TetRec r;
+      float row[kIncidentRow];
+#pragma unroll
+      for (int i = 0; i < kIncidentRow; ++i) row[i] = 0.0f;
+      if (incidentTetChecked(b.tets, entry, b.tetTotal, b.vertexTotal, &r)) {
+        const M3 F = deformationAt(r, x);
+        const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
+        const float3 g = shapeGradient(r, entry & 3u);
+        const float3 f = r.vol * mv(piola(F, pt), g);
+        row[0] = f.x; row[1] = f.y; row[2] = f.z;
+        if (kHessian) {
+          const S3 blk = incidentBlock(r, F, pt, g);
+          row[3] = blk.xx; row[4] = blk.yy; row[5] = blk.zz; row[6] = blk.xy; row[7] = blk.xz; row[8] = blk.yz;
+        }
+        row[9] = F.c0.x; row[10] = F.c0.y; row[11] = F.c0.z;
+        row[12] = F.c1.x; row[13] = F.c1.y; row[14] = F.c1.z;
+        row[15] = F.c2.x; row[16] = F.c2.y; row[17] = F.c2.z;
+        row[18] = 1.0f;
+        row[19] = r.vol;
+      }
+      float4* dst = reinterpret_cast<float4*>(rows + lane * kIncidentRow);
+#pragma unroll
+      for (int i = 0; i < kIncidentRow / 4; ++i)
+        dst[i] = make_float4(row[4 * i], row[4 * i + 1], row[4 * i + 2], row[4 * i + 3]);
+    }
+    __syncwarp(mask);
+    for (uint32_t j = 0; j < n; ++j) {
+      const float* q = rows + j * kIncidentRow;
+      const float vol = q[19];
+      if (lane < 3) {
+        float e;
+        s[0] = twoSum(s[0], q[lane], &e);
+        c = __fadd_rn(c, e);
+      } else {
+        s[0] = __fmaf_rn(vol, q[lane], s[0]);
+      }
+      s[1] = __fmaf_rn(vol, q[8 + lane], s[1]);
+      if (lane < 3) s[2] = __fmaf_rn(vol, q[16 + lane], s[2]);
+    }
+    __syncwarp(mask);
+  }
+  out[lane] = s[0];
+  out[8 + lane] = s[1];
+  if (lane < 3) {
+    out[16 + lane] = s[2];
+    out[19 + lane] = c;
+  }
+}
+__device__ __forceinline__ IncidentSums loadIncidentSums(const float* q) {
+  IncidentSums o;
+  o.grad.s = f3(q[0], q[1], q[2]);
+  o.grad.c = f3(q[19], q[20], q[21]);
+  o.hess = {q[3], q[4], q[5], q[6], q[7], q[8]};
+  o.avg = {f3(q[9], q[10], q[11]), f3(q[12], q[13], q[14]), f3(q[15], q[16], q[17])};
+  o.total = q[18];
+  return o;
+}
+// The sums of an entry's (at most 32) vertices, eight lanes per vertex, left
+// in shared memory (ends with a block barrier).
+__device__ __forceinline__ void incidentBlockSums(const Buffers& b, const float4* __restrict__ x, const RedBlock& rb,
+                                                  const SceneRange& sr, bool pinnedToo, IncidentShared& sh) {
+  const uint32_t group = threadIdx.x / kIncidentLanes, k = rb.begin + group;
+  if (k < rb.end) {
+    const uint4 info = b.vinfo[sr.vOff + k];
+    if (pinnedToo || !isPinned(info))
+      incidentSumsLanes<true>(b, x, info, reinterpret_cast<float*>(sh.rows4) + group * kIncidentGroup,
+                              threadIdx.x % kIncidentLanes, 0xffu << (threadIdx.x & 24u), sh.sums[group]);
+  }
+  __syncthreads();
+}
+
+// Cloth terms, frame and incident system of a free vertex from its sums: the
+// frame is the polar of the volume-weighted average F (vertexPolarRotation,
+// jgs2-shader.ts:2959-2989), the system the incident material gradient and
+// Hessian blocks plus the membrane and bending terms of the vertex's cloth.
+__device__ __forceinline__ void storeFrameAndIncident(const Buffers& b, const DevParams& p,
+                                                      const float4* __restrict__ x, uint32_t v, const uint4& info,
+                                                      IncidentSums& o) {
   if (p.cloth)
     clothLocalSystem<true>(b.clothTris, b.clothHinges, b.clothIncidence, b.clothRange[v], x, clothMaterial(p), 0u, 1u,
-                           grad, hess);
-  const M3 favg = total > 0.0f ? (1.0f / total) * avg : midentity();
-  storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, eps));
-  storeIncident(b.incident, v, cvalue(grad), hess);
+                           o.grad, o.hess);
+  const M3 favg = o.total > 0.0f ? (1.0f / o.total) * o.avg : midentity();
+  storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
+  storeIncident(b.incident, v, cvalue(o.grad), o.hess);
 }
 
 // Vertex frame: polar of the volume-weighted average F over incident tets
@@ -2456,10 +2571,9 @@ __global__ void __launch_bounds__(kBlock, JGS2_SOLVE_MIN_BLOCKS)
 }
 
 // ---------------------------------------------------------------------------
-// Grid-wide reductions.  Each of the prologue, gate and convergence kernels
-// runs on a persistent grid (a few blocks per SM, grid-stride loops), folds
-// its elements into one partial per block with a fixed tree, writes the
-// partial, and the last block to take a ticket folds all partials in block
+// Grid-wide reductions.  The gate's blocks and the prologue's and the
+// convergence pass's warps each fold their elements into one partial with a
+// fixed tree; the last to take a ticket folds the scene's partials in a fixed
 // order.  Results are deterministic for a given device; nothing waits.
 struct GatePartial {
   double e0, e1;      // source / candidate assembled energy
@@ -2501,17 +2615,44 @@ __device__ __forceinline__ void convCombine(ConvPartial& a, const ConvPartial& b
   a.valid &= b.valid;
 }
 
-template <class P, class C>
-__device__ __forceinline__ P blockFold(P v, P* smem, C combine) {
-  smem[threadIdx.x] = v;
-  __syncthreads();
-  for (unsigned s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) combine(smem[threadIdx.x], smem[threadIdx.x + s]);
-    __syncthreads();
-  }
-  P r = smem[0];
-  __syncthreads();
+// One value from the other lane of a shuffle step, word by word.
+template <class P>
+__device__ __forceinline__ P shflDown(const P& v, unsigned offset) {
+  static_assert(sizeof(P) % 4 == 0, "partials are moved as 32-bit words");
+  uint32_t words[sizeof(P) / 4];
+  memcpy(words, &v, sizeof(P));
+#pragma unroll
+  for (unsigned i = 0; i < sizeof(P) / 4; ++i) words[i] = __shfl_down_sync(0xffffffffu, words[i], offset);
+  P r;
+  memcpy(&r, words, sizeof(P));
   return r;
+}
+
+// Warp value in lane 0 (fixed tree).
+template <class P, class C>
+__device__ __forceinline__ P warpFold(P v, C combine) {
+#pragma unroll
+  for (unsigned o = 16; o > 0; o >>= 1) combine(v, shflDown(v, o));
+  return v;
+}
+
+// Block value in thread 0 (fixed tree: lanes by shuffles, then the warps'
+// values in one more shuffle tree).  `smem` holds one value per warp.  A tree
+// in shared memory took a block barrier per level, seven at 128 threads, and
+// blocks of small scenes do little else.
+template <class P, class I, class C>
+__device__ __forceinline__ P blockFold(P v, P* smem, I identity, C combine) {
+  v = warpFold(v, combine);
+  const unsigned warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
+  if (lane == 0) smem[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    v = lane < kBlock / 32 ? smem[lane] : identity();
+#pragma unroll
+    for (unsigned o = kBlock / 64; o > 0; o >>= 1) combine(v, shflDown(v, o));
+  }
+  __syncthreads();
+  return v;
 }
 
 // Publishes the block partial at `slot`; returns true in every thread of the
@@ -2530,22 +2671,75 @@ __device__ __forceinline__ bool publishPartial(const P& blockValue, P* partials,
   return last;
 }
 
-// Folds partials[0, count) in index order (deterministic).
+// Partials first, first + stride, ... below count, added in that order.
+// Other blocks wrote them: they are read from L2, four of a thread's in
+// flight at a time (one at a time, the 2 930 gate partials of six million
+// tets kept the last block waiting for 23 L2 round trips).
+template <class P, class C>
+__device__ __forceinline__ void addPartials(P& acc, const P* partials, uint32_t first, uint32_t stride, uint32_t count,
+                                            C combine) {
+  static_assert(sizeof(P) % 16 == 0, "partials are read as 16-byte words");
+  constexpr uint32_t kAhead = 4, kWords = sizeof(P) / 16;
+  for (uint32_t k0 = first; k0 < count; k0 += stride * kAhead) {
+    uint4 words[kAhead][kWords];
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) {
+      const uint4* w = reinterpret_cast<const uint4*>(partials + min(k0 + stride * j, count - 1));
+#pragma unroll
+      for (uint32_t i = 0; i < kWords; ++i) words[j][i] = __ldcg(w + i);
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) {
+      P v;
+      memcpy(&v, words[j], sizeof(P));
+      if (k0 + stride * j < count) combine(acc, v);
+    }
+  }
+}
+
+// Folds partials[0, count) by a block (deterministic).
 template <class P, class I, class C>
 __device__ __forceinline__ P foldPartials(const P* partials, uint32_t count, P* smem, I identity, C combine) {
   P acc = identity();
-  static_assert(sizeof(P) % 4 == 0, "partials are read as 32-bit words");
-  for (uint32_t k = threadIdx.x; k < count; k += blockDim.x) {
-    // Other blocks wrote these partials: read them from L2.
-    uint32_t words[sizeof(P) / 4];
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(partials + k);
-#pragma unroll
-    for (unsigned i = 0; i < sizeof(P) / 4; ++i) words[i] = __ldcg(w + i);
-    P v;
-    memcpy(&v, words, sizeof(P));
-    combine(acc, v);
-  }
-  return blockFold(acc, smem, combine);
+  addPartials(acc, partials, threadIdx.x, blockDim.x, count, combine);
+  return blockFold(acc, smem, identity, combine);
+}
+
+// Reduction over entries of one warp each (prologue and convergence): the
+// last warp of 32 consecutive entries folds them into the group's partial and
+// the last of those folds the scene's groups, so no warp reads more than a
+// few partials per lane.  True, with the scene's value in lane 0 of `value`,
+// on the scene's last warp; the tickets are then zero again.
+template <class P, class I, class C>
+__device__ __forceinline__ bool foldEntries(P& value, P* partials, P* groups, uint32_t* groupTickets,
+                                            uint32_t* ticket, const RedBlock& rb, const SceneRange& sr, I identity,
+                                            C combine) {
+  const uint32_t lane = threadIdx.x & 31u;
+  auto publish = [&](P* at, uint32_t* t, uint32_t count) {
+    uint32_t last = 0;
+    if (lane == 0) {
+      *at = value;
+      __threadfence();
+      last = atomicAdd(t, 1u) == count - 1 ? 1u : 0u;
+      if (last) *t = 0u;
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (last) __threadfence();
+    return last != 0u;
+  };
+  value = warpFold(value, combine);
+  const uint32_t local = rb.slot - sr.convBase, group = local / 32, first = group * 32;
+  const uint32_t inGroup = min(32u, sr.convBlocks - first), groupCount = (sr.convBlocks + 31) / 32;
+  if (!publish(&partials[rb.slot], &groupTickets[sr.convGroupBase + group], inGroup)) return false;
+  P acc = identity();
+  addPartials(acc, partials + sr.convBase + first, lane, 32u, inGroup, combine);
+  value = warpFold(acc, combine);
+  if (groupCount == 1) return true;
+  if (!publish(&groups[sr.convGroupBase + group], ticket, groupCount)) return false;
+  acc = identity();
+  addPartials(acc, groups + sr.convGroupBase, lane, 32u, groupCount, combine);
+  value = warpFold(acc, combine);
+  return true;
 }
 
 __device__ __forceinline__ void accumulateTet(GatePartial& acc, const TetRec& r, const M3& sF, const M3& cF) {
@@ -2635,63 +2829,91 @@ __device__ __forceinline__ void accumulateHinge(GatePartial& acc, const float4* 
 // Prologue: predict (jgs2-shader.ts:2660-2692), iteration-0 vertex frames and
 // the source feasibility preflight (candidateTetrahedron + reduceCandidate on
 // the accepted pose, jgs2-solver.ts:2240-2259).
-__global__ void __launch_bounds__(kBlock) prologueKernel(Buffers b, const DevParams* __restrict__ pp) {
-  __shared__ GatePartial smem[kBlock];
-  __shared__ bool isLast;
-  const RedBlock rb = b.gateTable[blockIdx.x];
+// Elements [x, y) of `n` that fall to a scene's convergence block.
+__device__ __forceinline__ uint2 blockShare(uint32_t n, const RedBlock& rb, const SceneRange& sr) {
+  const uint64_t i = rb.slot - sr.convBase;
+  return make_uint2(static_cast<uint32_t>(n * i / sr.convBlocks), static_cast<uint32_t>(n * (i + 1) / sr.convBlocks));
+}
+
+// One warp per reduction entry: its vertices, and its share of the scene's
+// tets, cloth triangles and hinges, so every warp has the same mix of work.
+// kWide: a block per entry, whose eight warps first form the incident sums.
+template <bool kWide>
+__global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) prologueKernel(Buffers b,
+                                                                              const DevParams* __restrict__ pp) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t entry = kWide ? blockIdx.x : blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
+  if (entry >= b.convBlocks) return;  // uniform across the warp
+  const RedBlock rb = b.convTable[entry];
   const SceneRange sr = b.scenes[rb.scene];
   const DevParams p = pp[rb.scene];
-  if (!p.active) return;  // uniform across the scene's blocks
+  if (!p.active) return;  // uniform across the scene's entries
   FrameState* fs = &b.frames[rb.scene];
   GatePartial acc = gateIdentity();
-  for (uint32_t k = rb.begin + threadIdx.x; k < rb.end; k += blockDim.x) {
-    if (k < sr.V) {
-      const uint32_t i = sr.vOff + k;
-      const float4 o = b.pos[0][i];
-      b.old[i] = make_float4(o.x, o.y, o.z, 1.0f);
-      const uint4 info = b.vinfo[i];
-      const float4 rm = b.restMass[i];
-      float3 pred = xyz(rm);
-      if (!isPinned(info)) {
-        const float3 vel = p.velocityDamping * xyz(b.velocity[i]);
-        pred = xyz(o) + p.dt * vel + (p.dt * p.dt) * f3(p.gravity[0], p.gravity[1], p.gravity[2]);
-      } else {
-        b.velocity[i] = make_float4(0, 0, 0, 0);
-      }
-      b.predicted[i] = make_float4(pred.x, pred.y, pred.z, distributedInertiaWeight(rm, info, p.invDt2));
-      b.finalUpdate[i] = 0.0f;
-      if (!p.globalization) {
-        // Co-rotated path: the iteration source is the inertial prediction.
-        b.pos[1][i] = make_float4(pred.x, pred.y, pred.z, 1.0f);
-        continue;
-      }
-      // The stable iteration source is the accepted pose.
-      b.pos[1][i] = make_float4(o.x, o.y, o.z, 1.0f);
-      // Iteration-0 frames (and, for free vertices, the incident system).
-      if (isPinned(info)) storeFrame(b.vertexRot, i, vertexFrame(b, b.pos[0], i, p.rotationEpsilon));
-      else frameAndIncident(b, p, b.pos[0], i, info, p.rotationEpsilon);
-      const float e = implicitEnergy(p, b, i, xyz(o), info);
-      if (finiteS(e)) { acc.e0 += e; acc.e1 += e; }
-      else acc.bits &= ~(kSourceEnergyValid | kCandidateEnergyValid);
+  IncidentShared* sh = nullptr;
+  if constexpr (kWide) {
+    __shared__ IncidentShared shared;
+    sh = &shared;
+    if (p.globalization) incidentBlockSums(b, b.pos[0], rb, sr, true, shared);
+    if (threadIdx.x >= 32) return;
+  }
+  for (uint32_t k = rb.begin + lane; k < rb.end; k += 32) {
+    const uint32_t i = sr.vOff + k;
+    const float4 o = b.pos[0][i];
+    b.old[i] = make_float4(o.x, o.y, o.z, 1.0f);
+    const uint4 info = b.vinfo[i];
+    const float4 rm = b.restMass[i];
+    float3 pred = xyz(rm);
+    if (!isPinned(info)) {
+      const float3 vel = p.velocityDamping * xyz(b.velocity[i]);
+      pred = xyz(o) + p.dt * vel + (p.dt * p.dt) * f3(p.gravity[0], p.gravity[1], p.gravity[2]);
+    } else {
+      b.velocity[i] = make_float4(0, 0, 0, 0);
     }
-    if (p.globalization && k < sr.T) {
+    b.predicted[i] = make_float4(pred.x, pred.y, pred.z, distributedInertiaWeight(rm, info, p.invDt2));
+    b.finalUpdate[i] = 0.0f;
+    // Co-rotated path: the iteration source is the inertial prediction; the
+    // stable iteration source is the accepted pose.
+    const float3 first = p.globalization ? xyz(o) : pred;
+    b.pos[1][i] = make_float4(first.x, first.y, first.z, 1.0f);
+    if (!p.globalization) continue;
+    // Iteration-0 frames (and, for free vertices, the incident system).
+    IncidentSums sums = incidentZero();
+    if constexpr (kWide) sums = loadIncidentSums(sh->sums[k - rb.begin]);
+    else incidentSums<true>(b, b.pos[0], info, sums);
+    if (isPinned(info)) {
+      const M3 favg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
+      storeFrame(b.vertexRot, i, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
+    } else {
+      storeFrameAndIncident(b, p, b.pos[0], i, info, sums);
+    }
+    const float e = implicitEnergy(p, b, i, xyz(o), info);
+    if (finiteS(e)) { acc.e0 += e; acc.e1 += e; }
+    else acc.bits &= ~(kSourceEnergyValid | kCandidateEnergyValid);
+  }
+  if (p.globalization) {
+    const uint2 tets = blockShare(sr.T, rb, sr);
+    for (uint32_t k = tets.x + lane; k < tets.y; k += 32) {
       const TetRec r = loadTet(b.tets, sr.tOff + k);
       if (tetVerticesInBounds(r.idx, b.vertexTotal)) {
         const M3 F = deformationAt(r, b.pos[0]);
         accumulateTet(acc, r, F, F);
       }
     }
-    if (p.cloth) {
-      if (k < sr.C) accumulateClothTri(acc, loadClothTri(b.clothTris, sr.cOff + k), b.pos[0], b.pos[0], clothMaterial(p));
-      if (k < sr.H) accumulateHinge(acc, b.clothHinges, sr.hOff + k, b.pos[0], b.pos[0], p.clothBending);
-    }
+  }
+  if (p.cloth) {
+    const uint2 tris = blockShare(sr.C, rb, sr), hinges = blockShare(sr.H, rb, sr);
+    for (uint32_t k = tris.x + lane; k < tris.y; k += 32)
+      accumulateClothTri(acc, loadClothTri(b.clothTris, sr.cOff + k), b.pos[0], b.pos[0], clothMaterial(p));
+    for (uint32_t k = hinges.x + lane; k < hinges.y; k += 32)
+      accumulateHinge(acc, b.clothHinges, sr.hOff + k, b.pos[0], b.pos[0], p.clothBending);
   }
   if (!p.globalization) return;  // no preflight on the co-rotated path (uniform)
-  const GatePartial blk = blockFold(acc, smem, gateCombine);
-  GatePartial* partials = reinterpret_cast<GatePartial*>(b.gatePartials);
-  if (!publishPartial(blk, partials, rb.slot, sr.gateBlocks, &fs->prologueTicket, &isLast)) return;
-  const GatePartial tot = foldPartials(partials + sr.gateBase, sr.gateBlocks, smem, gateIdentity, gateCombine);
-  if (threadIdx.x != 0) return;
+  GatePartial tot = acc;
+  if (!foldEntries(tot, reinterpret_cast<GatePartial*>(b.gatePartials), reinterpret_cast<GatePartial*>(b.groupPartials),
+                   b.groupTickets, &fs->prologueTicket, rb, sr, gateIdentity, gateCombine))
+    return;
+  if (lane != 0) return;
   uint32_t vb = tot.bits;
   if (sr.T == 0) vb &= ~(kSourceGeometryValid | kCandidateGeometryValid);
   const bool gv = (vb & kSourceGeometryValid) != 0u;
@@ -2707,7 +2929,6 @@ __global__ void __launch_bounds__(kBlock) prologueKernel(Buffers b, const DevPar
   fs->control[1] = make_float4(accepted ? 1.f : 0.f, accepted ? 0.f : 1.f, 0.f, 0.f);
   fs->control[2] = make_float4(ev ? e0 : 0.f, ev ? e0 : 0.f, ev ? e0 : 0.f, ev ? 1.f : 0.f);
   fs->control[3] = make_float4(0, 0, 0, 0);
-  fs->prologueTicket = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -2732,7 +2953,7 @@ template <bool kExt>
 __global__ void __launch_bounds__(kBlock, kExt ? JGS2_GATE_EXT_MIN_BLOCKS : JGS2_GATE_MIN_BLOCKS)
     gateKernel(Buffers b, const DevParams* __restrict__ pp, const float4* __restrict__ src,
                const float4* __restrict__ tgt) {
-  __shared__ GatePartial smem[kBlock];
+  __shared__ GatePartial smem[kBlock / 32];
   __shared__ bool isLast;
   const RedBlock rb = b.gateTable[blockIdx.x];
   const SceneRange sr = b.scenes[rb.scene];
@@ -2766,7 +2987,7 @@ __global__ void __launch_bounds__(kBlock, kExt ? JGS2_GATE_EXT_MIN_BLOCKS : JGS2
       for (uint32_t c = k; c < contacts.y; c += span)
         accumulateContact(acc, b, p, fs->contactAlpha, contacts.x + c, src, tgt);
   }
-  const GatePartial blk = blockFold(acc, smem, gateCombine);
+  const GatePartial blk = blockFold(acc, smem, gateIdentity, gateCombine);
   GatePartial* partials = reinterpret_cast<GatePartial*>(b.gatePartials);
   if (!publishPartial(blk, partials, rb.slot, sr.gateBlocks, &fs->gateTicket, &isLast)) return;
   const GatePartial tot = foldPartials(partials + sr.gateBase, sr.gateBlocks, smem, gateIdentity, gateCombine);
@@ -2813,33 +3034,38 @@ __global__ void __launch_bounds__(kBlock, kExt ? JGS2_GATE_EXT_MIN_BLOCKS : JGS2
 // The five component norms are exact Euclidean norms accumulated in double;
 // the reference forms the same norms in f32 as scale * sqrt(sum((g/scale)^2)).
 // JGS2_CONV_MIN_BLOCKS: blocks per SM the convergence kernel's register
-// budget must allow (0: the compiler's choice, 151 registers and 3 blocks).
+// budget must allow (the compiler's choice is 151 registers and 3 blocks).
 // Four blocks (128 registers) measured 5 % faster on the 100^3 cube than the
 // compiler's choice, with bitwise the same results; five and six were slower.
 #ifndef JGS2_CONV_MIN_BLOCKS
 #define JGS2_CONV_MIN_BLOCKS 4
 #endif
-#if JGS2_CONV_MIN_BLOCKS > 0
-#define JGS2_CONV_BOUNDS __launch_bounds__(kBlock, JGS2_CONV_MIN_BLOCKS)
-#else
-#define JGS2_CONV_BOUNDS __launch_bounds__(kBlock)
-#endif
-
-__global__ void JGS2_CONV_BOUNDS convergenceKernel(Buffers b, const DevParams* __restrict__ pp,
-                                                            const float4* __restrict__ src, float4* tgt,
-                                                            int nextRotations) {
-  __shared__ ConvPartial smem[kBlock];
-  __shared__ bool isLast;
-  const RedBlock rb = b.convTable[blockIdx.x];
+// One warp per reduction entry.  kWide: a block per entry, whose eight warps
+// first form the incident sums; then the first warp goes on alone.
+template <bool kWide>
+__global__ void __launch_bounds__(kWide ? kWideBlock : kBlock, kWide ? 2 : JGS2_CONV_MIN_BLOCKS)
+    convergenceKernel(Buffers b, const DevParams* __restrict__ pp, const float4* __restrict__ src, float4* tgt,
+                      int nextRotations) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t entry = kWide ? blockIdx.x : blockIdx.x * (kBlock / 32) + threadIdx.x / 32;
+  if (entry >= b.convBlocks) return;  // uniform across the warp
+  const RedBlock rb = b.convTable[entry];
   const SceneRange sr = b.scenes[rb.scene];
   const DevParams p = pp[rb.scene];
   FrameState* fs = &b.frames[rb.scene];
-  if (!p.active || latched(p, fs)) return;  // uniform across the scene's blocks
+  if (!p.active || latched(p, fs)) return;  // uniform across the scene's entries
   const bool accepted = fs->control[1].x == 1.0f;
   const float4* __restrict__ acc = accepted ? tgt : src;
   const uint32_t V = sr.V;
   ConvPartial part = convIdentity();
-  for (uint32_t k = rb.begin + threadIdx.x; k < rb.end; k += blockDim.x) {
+  IncidentShared* sh = nullptr;
+  if constexpr (kWide) {
+    __shared__ IncidentShared shared;
+    sh = &shared;
+    incidentBlockSums(b, acc, rb, sr, nextRotations != 0, shared);
+    if (threadIdx.x >= 32) return;
+  }
+  for (uint32_t k = rb.begin + lane; k < rb.end; k += 32) {
     const uint32_t v = sr.vOff + k;
     float upd = 0.0f;
     if (!accepted) {
@@ -2850,45 +3076,18 @@ __global__ void JGS2_CONV_BOUNDS convergenceKernel(Buffers b, const DevParams* _
     b.finalUpdate[v] = upd;
     if (!(finiteS(upd) && upd >= 0.0f)) part.valid = 0u; else part.maxUpdate = fmaxf(part.maxUpdate, upd);
     const uint4 info = b.vinfo[v];
+    IncidentSums sums = incidentZero();
+    if (nextRotations || !isPinned(info)) {
+      if constexpr (kWide) sums = loadIncidentSums(sh->sums[k - rb.begin]);
+      else if (nextRotations) incidentSums<true>(b, acc, info, sums);
+      else incidentSums<false>(b, acc, info, sums);
+    }
     if (!isPinned(info)) {
       const float3 x = xyz(acc[v]);
       float3 comps[5];
       comps[0] = (b.restMass[v].w * p.invDt2) * (x - xyz(b.predicted[v]));
-      Comp3 material = czero();  // compensated gradient gather
-      M3 avg = mzero();
-      float total = 0.0f;
-      S3 hess = szero();
-#if JGS2_CONV_LOOKAHEAD
-      // The next incident tet's record is requested before the current
-      // one's arithmetic, so its latency overlaps the work.
-      uint32_t nextEntry = info.y ? __ldg(&b.adjacency[info.x]) : 0u;
-      TetRec nextRec;
-      bool nextOk = false;
-  if (info.y) nextOk = incidentTetChecked(b.tets, nextEntry, b.tetTotal, b.vertexTotal, &nextRec);
-#endif
-      for (uint32_t a = 0; a < info.y; ++a) {
-#if JGS2_CONV_LOOKAHEAD
-        const uint32_t entry = nextEntry;
-        const TetRec r = nextRec;
-        const bool tetOk = nextOk;
-        if (a + 1 < info.y) {
-          nextEntry = __ldg(&b.adjacency[info.x + a + 1]);
-          nextOk = incidentTetChecked(b.tets, nextEntry, b.tetTotal, b.vertexTotal, &nextRec);
-        }
-#else
-        const uint32_t entry = __ldg(&b.adjacency[info.x + a]);
-        TetRec r;
-        const bool tetOk = incidentTetChecked(b.tets, entry, b.tetTotal, b.vertexTotal, &r);
-#endif
-        if (!tetOk) continue;
-        const M3 F = deformationAt(r, acc);
-        const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
-        const float3 g = shapeGradient(r, entry & 3u);
-        cadd(material, r.vol * mv(piola(F, pt), g));
-        if (nextRotations) addIncidentBlock(hess, r, F, pt, g);
-        avg = avg + r.vol * F;
-        total += r.vol;
-      }
+      Comp3& material = sums.grad;
+      S3& hess = sums.hess;
       if (p.cloth) {
         const uint4 cr = b.clothRange[v];
         if (nextRotations)
@@ -2931,20 +3130,18 @@ __global__ void JGS2_CONV_BOUNDS convergenceKernel(Buffers b, const DevParams* _
       }
       // The next iteration's frame and incident system from the same
       // deformation gradients (the accepted pose is the next source).
-      if (nextRotations) {
-        const M3 favg = total > 0.0f ? (1.0f / total) * avg : midentity();
-        storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
-        storeIncident(b.incident, v, comps[1], hess);
-      }
-    } else if (nextRotations) {
-      storeFrame(b.vertexRot, v, vertexFrame(b, acc, v, p.rotationEpsilon));
+      if (nextRotations) storeIncident(b.incident, v, comps[1], hess);
+    }
+    if (nextRotations) {
+      const M3 favg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
+      storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
     }
   }
-  const ConvPartial blk = blockFold(part, smem, convCombine);
-  ConvPartial* partials = reinterpret_cast<ConvPartial*>(b.convPartials);
-  if (!publishPartial(blk, partials, rb.slot, sr.convBlocks, &fs->convTicket, &isLast)) return;
-  const ConvPartial tot = foldPartials(partials + sr.convBase, sr.convBlocks, smem, convIdentity, convCombine);
-  if (threadIdx.x != 0) return;
+  ConvPartial tot = part;
+  if (!foldEntries(tot, reinterpret_cast<ConvPartial*>(b.convPartials), reinterpret_cast<ConvPartial*>(b.groupPartials),
+                   b.groupTickets, &fs->convTicket, rb, sr, convIdentity, convCombine))
+    return;
+  if (lane != 0) return;
   float norms[5];
   bool cnv = tot.valid != 0u;
   for (int c = 0; c < 5; ++c) {
@@ -2993,7 +3190,6 @@ __global__ void JGS2_CONV_BOUNDS convergenceKernel(Buffers b, const DevParams* _
   }
   fs->control[1].w = float(hi + 1);
   if (conv && p.stopEnabled) fs->control[0].w = float(cb | kStopLatchBit);
-  fs->convTicket = 0u;
 }
 
 // ---------------------------------------------------------------------------
@@ -3075,7 +3271,7 @@ __global__ void __launch_bounds__(kBlock) gateScratchKernel(Buffers b, DevParams
                                                             const float4* __restrict__ tgt, uint32_t V, uint32_t T,
                                                             uint32_t C, uint32_t H, float4* __restrict__ control,
                                                             unsigned char* __restrict__ scratch) {
-  __shared__ GatePartial smem[kBlock];
+  __shared__ GatePartial smem[kBlock / 32];
   __shared__ bool isLast;
   uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch);
   GatePartial* partials = reinterpret_cast<GatePartial*>(scratch + kGateScratchHeaderBytes);
@@ -3094,7 +3290,7 @@ __global__ void __launch_bounds__(kBlock) gateScratchKernel(Buffers b, DevParams
   }
   if (i < C) accumulateClothTri(acc, loadClothTri(b.clothTris, i), src, tgt, clothMaterial(p));
   if (i < H) accumulateHinge(acc, b.clothHinges, i, src, tgt, p.clothBending);
-  const GatePartial blk = blockFold(acc, smem, gateCombine);
+  const GatePartial blk = blockFold(acc, smem, gateIdentity, gateCombine);
   if (!publishPartial(blk, partials, blockIdx.x, gridDim.x, ticket, &isLast)) return;
   const GatePartial tot = foldPartials(partials, gridDim.x, smem, gateIdentity, gateCombine);
   if (threadIdx.x != 0) return;
@@ -3357,8 +3553,19 @@ uint32_t smCount() {
   return static_cast<uint32_t>(sms);
 }
 
+// Eight lanes per vertex in the prologue and convergence passes, with the
+// same bits.  Measured per convergence launch (events, about 6 us of which is
+// the timing itself), eight lanes against one thread: 525 vertices 17 / 26 us,
+// 2 688 vertices 19 / 27, 13 392 vertices 29 / 31, 27 360 vertices 41 / 35,
+// 68 921 vertices 98 / 57: past about ten thousand vertices the threads hide
+// each other's gathers.  Cloth adds its triangles and hinges one thread per
+// vertex whichever way the tets are summed, so it keeps that form.
+constexpr uint32_t kWideVertices = 8192;
+bool wideIncident(const Buffers& b) { return b.vertexTotal <= kWideVertices && !b.clothRange; }
+
 int launchPrologue(const Buffers& b, const DevParams* p, cudaStream_t s) {
-  prologueKernel<<<b.gateBlocks, kBlock, 0, s>>>(b, p);
+  if (wideIncident(b)) prologueKernel<true><<<b.convBlocks, kWideBlock, 0, s>>>(b, p);
+  else prologueKernel<false><<<(b.convBlocks + kBlock / 32 - 1) / (kBlock / 32), kBlock, 0, s>>>(b, p);
   return 1;
 }
 
@@ -3649,7 +3856,10 @@ int launchGate(const Buffers& b, const DevParams* p, const float4* src, const fl
 
 int launchConvergence(const Buffers& b, const DevParams* p, const float4* src, float4* tgt,
                       bool computeNextRotations, cudaStream_t s) {
-  convergenceKernel<<<b.convBlocks, kBlock, 0, s>>>(b, p, src, tgt, computeNextRotations ? 1 : 0);
+  const int next = computeNextRotations ? 1 : 0;
+  if (wideIncident(b)) convergenceKernel<true><<<b.convBlocks, kWideBlock, 0, s>>>(b, p, src, tgt, next);
+  else
+    convergenceKernel<false><<<(b.convBlocks + kBlock / 32 - 1) / (kBlock / 32), kBlock, 0, s>>>(b, p, src, tgt, next);
   return 1;
 }
 

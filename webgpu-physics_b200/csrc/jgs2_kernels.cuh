@@ -43,14 +43,16 @@ struct DevParams {
 // of one scene.
 struct SceneRange {
   uint32_t vOff, V, tOff, T;
-  uint32_t gateBase, gateBlocks;  // prologue / gate partials of this scene
-  uint32_t convBase, convBlocks;  // convergence partials of this scene
+  uint32_t gateBase, gateBlocks;  // gate partials of this scene
+  uint32_t convBase, convBlocks;  // prologue and convergence partials of this scene
   uint32_t cOff, C, hOff, H;      // cloth triangles and hinges of this scene
   uint32_t kOff, KC;              // static IPC candidates of this scene
   uint32_t rowOff, rowCount;      // broad-phase rows of this scene (contact surface)
   // Elements one pass of the scene's gate blocks covers (the table's range);
   // broad-phase candidates beyond it stride over the same blocks.
-  uint32_t gateSpan, pad[3];
+  uint32_t gateSpan;
+  uint32_t convGroupBase;  // groups of 32 prologue / convergence entries of this scene
+  uint32_t pad[2];
 };
 
 // One block of a segmented reduction: elements [begin, end) of `scene`,
@@ -58,14 +60,20 @@ struct SceneRange {
 struct RedBlock {
   uint32_t scene, begin, end, slot;
 };
-#ifndef JGS2_GATE_CHUNK
-#define JGS2_GATE_CHUNK 2048
-#endif
-constexpr uint32_t kGateChunk = JGS2_GATE_CHUNK;  // tets / vertices per prologue or gate block
-#ifndef JGS2_CONV_CHUNK
-#define JGS2_CONV_CHUNK 256
-#endif
-constexpr uint32_t kConvChunk = JGS2_CONV_CHUNK;  // vertices per convergence block
+// Work split of the segmented passes, a function of the scene's own size so
+// that a scene folds the same partials alone and in a batch.
+//   Gate: 128 to 2 048 elements per block, about kGateBlocksPerScene blocks
+// for the sizes between.  At a fixed 2 048 elements a bar of 1 920 tets was
+// one block whose threads walked 16 elements one after another, two dependent
+// gathers each (gate of that bar 23.0 us, now 10.6; 148 074 tets 38.3 us, now
+// 14.6).  From 1.2 M elements on longer blocks fold fewer partials.
+//   Prologue and convergence: entries of kConvChunk vertices, one warp each.
+constexpr uint32_t kGateMinChunk = 128, kGateMaxChunk = 2048, kGateBlocksPerScene = 592;
+inline uint32_t gateChunk(uint32_t elements) {
+  const uint32_t per = (elements / kGateBlocksPerScene + kGateMinChunk - 1) / kGateMinChunk * kGateMinChunk;
+  return per < kGateMinChunk ? kGateMinChunk : per > kGateMaxChunk ? kGateMaxChunk : per;
+}
+constexpr uint32_t kConvChunk = 32;
 
 // Reduction scratch and the GPU-resident control/history records
 // (dynamic arena regions globalizationControl/globalizationHistory,
@@ -105,8 +113,10 @@ struct Buffers {
   // written by the pass that computes that pose's vertex frames.
   float4* incident;
   FrameState* frames;     // one per scene
-  void* gatePartials;     // one GatePartial (32 bytes) per gate / prologue block
-  void* convPartials;     // one ConvPartial (80 bytes) per convergence block
+  void* gatePartials;     // one GatePartial (32 bytes) per gate or prologue block
+  void* convPartials;     // one ConvPartial (80 bytes) per convergence entry
+  void* groupPartials;    // one partial of either kind per 32 entries
+  uint32_t* groupTickets; // arrivals per 32 entries, zero between passes
   double* bodyAccum;      // 6 per body (mass, solved xz, predicted xz, pinned count)
   // static
   const float4* restMass;     // rest xyz (pin target), mass
@@ -122,8 +132,8 @@ struct Buffers {
   const uint32_t* vertexScene;  // scene of each vertex
   const uint32_t* tetScene;     // scene of each tet (co-rotated engines only)
   const SceneRange* scenes;
-  const RedBlock* gateTable;    // prologue / gate blocks
-  const RedBlock* convTable;    // convergence blocks
+  const RedBlock* gateTable;    // gate blocks
+  const RedBlock* convTable;    // prologue and convergence blocks
   // Triangle cloth (all null when no scene has cloth): two float4 per
   // triangle (indices as uint + rest area, inverse rest basis), two per hinge
   // (indices as uint, rest angle and edge length), per vertex the incidence

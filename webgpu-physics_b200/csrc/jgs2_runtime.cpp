@@ -1931,6 +1931,7 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
   // Segmented reduction tables: each scene's elements in fixed chunks.
   std::vector<jgs2::SceneRange> ranges(S);
   std::vector<jgs2::RedBlock> gateTable, convTable;
+  uint32_t convGroups = 0;
   for (uint32_t i = 0; i < S; ++i) {
     const SceneHost& sc = sp->scenes[i];
     jgs2::SceneRange& r = ranges[i];
@@ -1945,13 +1946,16 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
     const uint32_t n = std::max(std::max(std::max(sc.V, sc.T), std::max(sc.C, sc.H)), std::max(sc.KC, listed));
     r.gateSpan = std::max(n, 1u);
     r.gateBase = static_cast<uint32_t>(gateTable.size());
-    for (uint32_t b0 = 0; b0 < std::max(n, 1u); b0 += jgs2::kGateChunk)
-      gateTable.push_back({i, b0, std::min(n, b0 + jgs2::kGateChunk), static_cast<uint32_t>(gateTable.size())});
+    const uint32_t gateChunk = jgs2::gateChunk(n);
+    for (uint32_t b0 = 0; b0 < std::max(n, 1u); b0 += gateChunk)
+      gateTable.push_back({i, b0, std::min(n, b0 + gateChunk), static_cast<uint32_t>(gateTable.size())});
     r.gateBlocks = static_cast<uint32_t>(gateTable.size()) - r.gateBase;
     r.convBase = static_cast<uint32_t>(convTable.size());
     for (uint32_t b0 = 0; b0 < std::max(sc.V, 1u); b0 += jgs2::kConvChunk)
       convTable.push_back({i, b0, std::min(sc.V, b0 + jgs2::kConvChunk), static_cast<uint32_t>(convTable.size())});
     r.convBlocks = static_cast<uint32_t>(convTable.size()) - r.convBase;
+    r.convGroupBase = convGroups;
+    convGroups += (r.convBlocks + 31) / 32;
   }
 
   jgs2_status st = JGS2_OK;
@@ -1997,10 +2001,15 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
   {
     double* gp = nullptr;
     double* cp = nullptr;
-    STEP(deviceAlloc(sp, &gp, jgs2::kGatePartialBytes / sizeof(double) * b.gateBlocks));
+    STEP(deviceAlloc(sp, &gp, jgs2::kGatePartialBytes / sizeof(double) * std::max(b.gateBlocks, b.convBlocks)));
     STEP(deviceAlloc(sp, &cp, jgs2::kConvPartialBytes / sizeof(double) * b.convBlocks));
     b.gatePartials = gp;
     b.convPartials = cp;
+    double* qp = nullptr;
+    STEP(deviceAlloc(sp, &qp, jgs2::kConvPartialBytes / sizeof(double) * convGroups));
+    b.groupPartials = qp;
+    STEP(deviceAlloc(sp, &b.groupTickets, convGroups));
+    CUDA_TRY(sp, cudaMemsetAsync(b.groupTickets, 0, sizeof(uint32_t) * convGroups, sp->stream));
     jgs2::RedBlock* gt = nullptr;
     jgs2::RedBlock* ct = nullptr;
     STEP(upload(sp, &gt, gateTable.data(), gateTable.size()));
