@@ -495,7 +495,9 @@ struct IncidentShared {
   float4 rows4[kConvChunk * kIncidentGroup / 4];
   float sums[kConvChunk][kIncidentSum];
 };
-template <bool kHessian>
+// What the sums are for: the frame alone, or the whole incident system too.
+enum IncidentPart { kFramePart, kSystemPart };
+template <IncidentPart kPart>
 __device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4* __restrict__ x, const uint4& info,
                                                   float* rows, uint32_t lane, unsigned mask, float* out) {
   float s[3] = {0.0f, 0.0f, 0.0f}, c = 0.0f;
@@ -509,11 +511,11 @@ __device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4
       for (int i = 0; i < kIncidentRow; ++i) row[i] = 0.0f;
       if (incidentTetChecked(b.tets, entry, b.tetTotal, b.vertexTotal, &r)) {
         const M3 F = deformationAt(r, x);
-        const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
-        const float3 g = shapeGradient(r, entry & 3u);
-        const float3 f = r.vol * mv(piola(F, pt), g);
-        row[0] = f.x; row[1] = f.y; row[2] = f.z;
-        if (kHessian) {
+        if constexpr (kPart == kSystemPart) {
+          const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
+          const float3 g = shapeGradient(r, entry & 3u);
+          const float3 f = r.vol * mv(piola(F, pt), g);
+          row[0] = f.x; row[1] = f.y; row[2] = f.z;
           const S3 blk = incidentBlock(r, F, pt, g);
           row[3] = blk.xx; row[4] = blk.yy; row[5] = blk.zz; row[6] = blk.xy; row[7] = blk.xz; row[8] = blk.yz;
         }
@@ -532,12 +534,14 @@ __device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4
     for (uint32_t j = 0; j < n; ++j) {
       const float* q = rows + j * kIncidentRow;
       const float vol = q[19];
-      if (lane < 3) {
-        float e;
-        s[0] = twoSum(s[0], q[lane], &e);
-        c = __fadd_rn(c, e);
-      } else {
-        s[0] = __fmaf_rn(vol, q[lane], s[0]);
+      if (kPart == kSystemPart) {
+        if (lane < 3) {
+          float e;
+          s[0] = twoSum(s[0], q[lane], &e);
+          c = __fadd_rn(c, e);
+        } else {
+          s[0] = __fmaf_rn(vol, q[lane], s[0]);
+        }
       }
       s[1] = __fmaf_rn(vol, q[8 + lane], s[1]);
       if (lane < 3) s[2] = __fmaf_rn(vol, q[16 + lane], s[2]);
@@ -568,7 +572,7 @@ __device__ __forceinline__ void incidentBlockSums(const Buffers& b, const float4
   if (k < rb.end) {
     const uint4 info = b.vinfo[sr.vOff + k];
     if (pinnedToo || !isPinned(info))
-      incidentSumsLanes<true>(b, x, info, reinterpret_cast<float*>(sh.rows4) + group * kIncidentGroup,
+      incidentSumsLanes<kSystemPart>(b, x, info, reinterpret_cast<float*>(sh.rows4) + group * kIncidentGroup,
                               threadIdx.x % kIncidentLanes, 0xffu << (threadIdx.x & 24u), sh.sums[group]);
   }
   __syncthreads();
@@ -608,17 +612,45 @@ __device__ __forceinline__ M3 vertexFrame(const Buffers& b, const float4* __rest
   return polarRotation(avg, eps);
 }
 
-// Vertex frames for a list of vertices (or all) from pose x.
-__global__ void __launch_bounds__(kBlock) vertexPolarKernel(Buffers b, const DevParams* __restrict__ pp,
-                                                            const float4* __restrict__ x,
-                                                            const uint32_t* __restrict__ list, uint32_t count) {
-  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= count) return;
-  const uint32_t v = list ? list[i] : i;
-  const uint32_t scene = b.vertexScene[v];
-  const DevParams& p = pp[scene];
-  if (!p.active || latched(p, &b.frames[scene])) return;
-  storeFrame(b.vertexRot, v, vertexFrame(b, x, v, p.rotationEpsilon));
+// Vertex frames for a list of vertices (or all) from pose x.  kWide: eight
+// lanes per vertex, 32 vertices a block, with the same bits, for lists of up
+// to kWideVertices (a colour of a 525-vertex bar: 18.6 us one thread per
+// vertex, 10.8 us so).
+template <bool kWide>
+__global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) vertexPolarKernel(Buffers b,
+                                                                                 const DevParams* __restrict__ pp,
+                                                                                 const float4* __restrict__ x,
+                                                                                 const uint32_t* __restrict__ list,
+                                                                                 uint32_t count) {
+  if constexpr (kWide) {
+    __shared__ IncidentShared sh;
+    const uint32_t group = threadIdx.x / kIncidentLanes, first = blockIdx.x * kConvChunk;
+    auto wanted = [&](uint32_t i, uint32_t* v) {
+      if (i >= count) return false;
+      *v = list ? list[i] : i;
+      const uint32_t scene = b.vertexScene[*v];
+      return pp[scene].active && !latched(pp[scene], &b.frames[scene]);
+    };
+    uint32_t v;
+    if (wanted(first + group, &v))
+      incidentSumsLanes<kFramePart>(b, x, b.vinfo[v], reinterpret_cast<float*>(sh.rows4) + group * kIncidentGroup,
+                                    threadIdx.x % kIncidentLanes, 0xffu << (threadIdx.x & 24u), sh.sums[group]);
+    __syncthreads();
+    if (threadIdx.x < kConvChunk && wanted(first + threadIdx.x, &v)) {
+      const IncidentSums sums = loadIncidentSums(sh.sums[threadIdx.x]);
+      const M3 avg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
+      storeFrame(b.vertexRot, v,
+                 b.vinfo[v].y == 0u ? midentity() : polarRotation(avg, pp[b.vertexScene[v]].rotationEpsilon));
+    }
+  } else {
+    const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+    if (i >= count) return;
+    const uint32_t v = list ? list[i] : i;
+    const uint32_t scene = b.vertexScene[v];
+    const DevParams& p = pp[scene];
+    if (!p.active || latched(p, &b.frames[scene])) return;
+    storeFrame(b.vertexRot, v, vertexFrame(b, x, v, p.rotationEpsilon));
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -646,10 +678,10 @@ __device__ __forceinline__ M3 stiffnessBlock(const float* __restrict__ k, uint32
   return {f3(r0[0], r1[0], r2[0]), f3(r0[1], r1[1], r2[1]), f3(r0[2], r1[2], r2[2])};
 }
 
-// Element gradient of a co-rotated tet at pose x (tetGradient):
-// R K (R^T (x_l - centroid) - (X_l - rest centroid)) per vertex slot.
-__device__ __forceinline__ void corotatedGradient(const Buffers& b, const float4* __restrict__ x, uint32_t t,
-                                                  const uint4& q, const M3& R, float3 out[4]) {
+// Displacements of a co-rotated tet's vertices in its frame,
+// R^T (x_l - centroid) - (X_l - rest centroid).
+__device__ __forceinline__ void corotatedDisplacement(const Buffers& b, const float4* __restrict__ x, const uint4& q,
+                                                      const M3& R, float3 disp[4]) {
   float3 cur[4], rest[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
@@ -660,46 +692,68 @@ __device__ __forceinline__ void corotatedGradient(const Buffers& b, const float4
   const float3 cc = 0.25f * (cur[0] + cur[1] + cur[2] + cur[3]);
   const float3 rc = 0.25f * (rest[0] + rest[1] + rest[2] + rest[3]);
   const M3 Rt = mtrans(R);
-  float3 disp[4];
 #pragma unroll
   for (int l = 0; l < 4; ++l) disp[l] = mv(Rt, cur[l] - cc) - (rest[l] - rc);
-  const float* k = b.stiffness + 144ull * t;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    float3 lg = f3(0, 0, 0);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) lg = lg + mv(stiffnessBlock(k, r, c), disp[c]);
-    out[r] = mv(R, lg);
-  }
 }
 
-// Reduced Hessian of a co-rotated record (cubatureHessian):
-// column c = sum_l B_l^T R K_l. R^T B_.[:, c].
-__device__ __forceinline__ M3 corotatedRecordHessian(const Buffers& b, uint32_t t, const M3& R, const M3 basis[4]) {
-  const M3 Rt = mtrans(R);
-  const float* k = b.stiffness + 144ull * t;
-  M3 out;
+// Block row `row` of a tet's rest stiffness: its four 3 x 3 blocks, from nine
+// vector loads.
+struct StiffnessRow {
+  M3 block[4];
+};
+__device__ __forceinline__ StiffnessRow stiffnessRow(const float* __restrict__ k, uint32_t row) {
+  const float4* q = reinterpret_cast<const float4*>(k) + 9u * row;
+  float f[3][12];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    float3 ld[4], wp[4];
+  for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int l = 0; l < 4; ++l) ld[l] = mv(Rt, c == 0 ? basis[l].c0 : (c == 1 ? basis[l].c1 : basis[l].c2));
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      float3 lp = f3(0, 0, 0);
-#pragma unroll
-      for (int cv = 0; cv < 4; ++cv) lp = lp + mv(stiffnessBlock(k, r, cv), ld[cv]);
-      wp[r] = mv(R, lp);
+    for (int j = 0; j < 3; ++j) {
+      const float4 v = __ldg(q + 3 * i + j);
+      f[i][4 * j] = v.x; f[i][4 * j + 1] = v.y; f[i][4 * j + 2] = v.z; f[i][4 * j + 3] = v.w;
     }
-    float3 col;
-    col.x = dot3(basis[0].c0, wp[0]) + dot3(basis[1].c0, wp[1]) + dot3(basis[2].c0, wp[2]) + dot3(basis[3].c0, wp[3]);
-    col.y = dot3(basis[0].c1, wp[0]) + dot3(basis[1].c1, wp[1]) + dot3(basis[2].c1, wp[2]) + dot3(basis[3].c1, wp[3]);
-    col.z = dot3(basis[0].c2, wp[0]) + dot3(basis[1].c2, wp[1]) + dot3(basis[2].c2, wp[2]) + dot3(basis[3].c2, wp[3]);
-    if (c == 0) out.c0 = col;
-    else if (c == 1) out.c1 = col;
-    else out.c2 = col;
+  StiffnessRow r;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    r.block[c] = {f3(f[0][3 * c], f[1][3 * c], f[2][3 * c]), f3(f[0][3 * c + 1], f[1][3 * c + 1], f[2][3 * c + 1]),
+                  f3(f[0][3 * c + 2], f[1][3 * c + 2], f[2][3 * c + 2])};
+  return r;
+}
+
+// R sum_c K_row,c d_c: a row of the element gradient (tetGradient) or of the
+// rotated stiffness times one basis column.
+__device__ __forceinline__ float3 stiffnessTimes(const StiffnessRow& row, const M3& R, const float3 d[4]) {
+  float3 lg = f3(0, 0, 0);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) lg = lg + mv(row.block[c], d[c]);
+  return mv(R, lg);
+}
+
+// Element gradient of a co-rotated record's tet and its reduced Hessian
+// (cubatureHessian), column c = sum_l B_l^T R K_l. R^T B_.[:, c], a block row of
+// the stiffness at a time so that each of its 144 floats is loaded once.
+__device__ __forceinline__ M3 corotatedRecordSystem(const float* __restrict__ k, const M3& R, const float3 disp[4],
+                                                    const M3 basis[4], float3 tg[4]) {
+  const M3 Rt = mtrans(R);
+  float3 ld[3][4];
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    ld[0][l] = mv(Rt, basis[l].c0);
+    ld[1][l] = mv(Rt, basis[l].c1);
+    ld[2][l] = mv(Rt, basis[l].c2);
   }
-  return out;
+  float3 col[3];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const StiffnessRow row = stiffnessRow(k, r);
+    tg[r] = stiffnessTimes(row, R, disp);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float3 wp = stiffnessTimes(row, R, ld[c]);
+      const float3 d = mtv(basis[r], wp);
+      col[c] = r == 0 ? d : col[c] + d;
+    }
+  }
+  return {col[0], col[1], col[2]};
 }
 
 // Distributed objective gradient / target stiffness of a record vertex.
@@ -709,104 +763,249 @@ __device__ __forceinline__ float3 distributedObjective(const DevParams& p, const
   return objectiveGradient(p, b, q, x) * (1.0f / float(qi.y > 1u ? qi.y : 1u));
 }
 
-// One thread per vertex: the exact co-rotated gather, the cubature
-// complement and the regularised solve (regularizedSolve, :2479-2512).
-__global__ void __launch_bounds__(kBlock) corotatedSolveKernel(Buffers b, const DevParams* __restrict__ pp,
-                                                               const float4* __restrict__ src, float4* tgt,
-                                                               const uint32_t* __restrict__ list, uint32_t count,
-                                                               uint32_t K) {
-  const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
-  if (i >= count) return;
-  const uint32_t v = list ? list[i] : i;
-  const DevParams& p = pp[b.vertexScene[v]];
-  if (!p.active) return;
+// The exact co-rotated gather, the cubature complement and the regularised
+// solve (regularizedSolve, :2479-2512) of kCoVertices vertices per block.
+// Every incident tet and every record is one thread's item: its gradient (3)
+// and Hessian (9) contribution goes to shared memory, then 12 threads per
+// vertex add one component each over the items in order (the vertex's own
+// terms, incident tets in adjacency order, floor, records in record order),
+// and one thread per vertex solves.  One thread per vertex for all of it, as
+// before, ran a chain of 24 tets and K records of 144-float stiffness
+// matrices serially: 322 us per launch at 1 200 vertices whatever the GPU had
+// idle.  The contributions and the order of the sums are the same, so are the
+// bits.
+#ifndef JGS2_CO_MIN_BLOCKS
+#define JGS2_CO_MIN_BLOCKS 2
+#endif
+constexpr uint32_t kCoVertices = 10;   // 120 component sums on 128 threads
+constexpr uint32_t kCoTets = 24;       // incident tets of a vertex per round
+constexpr uint32_t kCoRecords = 8;     // records of a vertex per round
+constexpr uint32_t kCoRow = 12;
+constexpr uint32_t kCoStride = (kCoTets + kCoRecords) * kCoRow + 12;  // floats per vertex: neighbours' sums read other banks
+
+// Contribution of cubature record `rec` of vertex v: w * projected gradient,
+// the projected Hessian and the weight (0 for an empty record).
+__device__ __forceinline__ float corotatedRecord(const Buffers& b, const DevParams& p, const float4* __restrict__ src,
+                                                 uint32_t v, size_t rec, float* row) {
+  const uint4 head = __ldg(&b.cubHead[2 * rec]);
+  const float w = __uint_as_float(head.y);
+  if (head.x == kEmptyTet || !(w > 0.0f)) return 0.0f;
   const uint4 info = b.vinfo[v];
-  const float4 rm = b.restMass[v];
-  if (isPinned(info)) {
-    tgt[v] = make_float4(rm.x, rm.y, rm.z, 1.0f);
-    b.finalUpdate[v] = 0.0f;
-    return;
-  }
   const float3 position = xyz(src[v]);
   const float4 pv = b.predicted[v];
-  const float inertia = rm.w * p.invDt2;
-  const bool objActive = p.objectiveFlags != 0u;
-  Comp3 gsum = czero();  // compensated gradient gather
-  cadd(gsum, inertia * (position - xyz(pv)));
-  M3 hess = inertia * midentity();
-  if (objActive) cadd(gsum, objectiveGradient(p, b, v, position));
-  if (p.objectiveFlags & 2u) hess = hess + targetStiffness(p, b, v) * midentity();
-  for (uint32_t a = 0; a < info.y; ++a) {
-    const uint32_t entry = __ldg(&b.adjacency[info.x + a]);
-    const uint32_t t = entry >> 2, slot = entry & 3u;
-    const TetRec r = loadTet(b.tets, t);
-    const M3 R = loadRot(b.tetRot, t);
-    float3 tg[4];
-    corotatedGradient(b, src, t, r.idx, R, tg);
-    cadd(gsum, tg[slot]);
-    hess = hess + mm(mm(R, stiffnessBlock(b.stiffness + 144ull * t, slot, slot)), mtrans(R));
-  }
-  if (p.floorStiffness > 0.0f && position.y < p.floorHeight) {
-    cadd(gsum, f3(0.0f, p.floorStiffness * (position.y - p.floorHeight), 0.0f));
-    hess.c1.y += p.floorStiffness;
-  }
-  const M3 RsT = mtrans(loadFrame(b.vertexRot, v));
   const float dWs = pv.w;
-  for (uint32_t s = 0; s < K; ++s) {
-    const size_t rec = static_cast<size_t>(v) * K + s;
-    const uint4 head = __ldg(&b.cubHead[2 * rec]);
-    const float w = __uint_as_float(head.y);
-    if (head.x == kEmptyTet || !(w > 0.0f)) continue;
-    const uint32_t t = head.x;
-    const uint4 q = __ldg(&b.cubHead[2 * rec + 1]);
-    const float4* U = b.cubBasis + 9ull * rec;
-    M3 basis[4];
+  const bool objActive = p.objectiveFlags != 0u;
+  const M3 RsT = mtrans(loadFrame(b.vertexRot, v));
+  const uint32_t t = head.x;
+  const uint4 q = __ldg(&b.cubHead[2 * rec + 1]);
+  const float4* U = b.cubBasis + 9ull * rec;
+  M3 basis[4];
 #pragma unroll
-    for (int l = 0; l < 4; ++l) basis[l] = mm(mm(loadFrame(b.vertexRot, idxAt(q, l)), loadBlockVec(U, l)), RsT);
-    const M3 R = loadRot(b.tetRot, t);
-    float3 tg[4];
-    corotatedGradient(b, src, t, q, R, tg);
-    float3 pg = f3(0, 0, 0);
-    M3 ih = mzero();
-    uint32_t ss = 4;
+  for (int l = 0; l < 4; ++l) basis[l] = mm(mm(loadFrame(b.vertexRot, idxAt(q, l)), loadBlockVec(U, l)), RsT);
+  const M3 R = loadRot(b.tetRot, t);
+  const float* k = b.stiffness + 144ull * t;
+  float3 disp[4], tg[4];
+  corotatedDisplacement(b, src, q, R, disp);
+  const M3 system = corotatedRecordSystem(k, R, disp, basis, tg);
+  float3 pg = f3(0, 0, 0);
+  M3 ih = mzero();
+  uint32_t ss = 4;
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const uint32_t qv = idxAt(q, l);
+    if (qv == v) ss = l;
+    const float4 pq = b.predicted[qv];
+    const float3 xq = xyz(src[qv]);
+    pg = pg + mtv(basis[l], tg[l] + pq.w * (xq - xyz(pq)));
+    ih = ih + pq.w * mm(mtrans(basis[l]), basis[l]);
+  }
+  if (objActive) {
 #pragma unroll
     for (int l = 0; l < 4; ++l) {
       const uint32_t qv = idxAt(q, l);
-      if (qv == v) ss = l;
-      const float4 pq = b.predicted[qv];
-      const float3 xq = xyz(src[qv]);
-      pg = pg + mtv(basis[l], tg[l] + pq.w * (xq - xyz(pq)));
-      ih = ih + pq.w * mm(mtrans(basis[l]), basis[l]);
+      pg = pg + mtv(basis[l], distributedObjective(p, b, qv, xyz(src[qv]), b.vinfo[qv]));
     }
-    if (objActive) {
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        const uint32_t qv = idxAt(q, l);
-        pg = pg + mtv(basis[l], distributedObjective(p, b, qv, xyz(src[qv]), b.vinfo[qv]));
-      }
-    }
-    M3 ph = corotatedRecordHessian(b, t, R, basis) + ih;
-    if (p.objectiveFlags & 2u) {
-      M3 oh = mzero();
-#pragma unroll
-      for (int l = 0; l < 4; ++l) {
-        const uint32_t qv = idxAt(q, l);
-        const uint4 qi = b.vinfo[qv];
-        const float kt = isPinned(qi) ? 0.0f : targetStiffness(p, b, qv) / float(qi.y > 1u ? qi.y : 1u);
-        oh = oh + kt * mm(mtrans(basis[l]), basis[l]);
-      }
-      ph = ph + oh;
-    }
-    if (ss < 4) {
-      pg = pg - (tg[ss] + dWs * (position - xyz(pv)));
-      if (objActive) pg = pg - distributedObjective(p, b, v, position, info);
-      ph = ph - (mm(mm(R, stiffnessBlock(b.stiffness + 144ull * t, ss, ss)), mtrans(R)) + dWs * midentity());
-      if (p.objectiveFlags & 2u)
-        ph = ph - (targetStiffness(p, b, v) / float(info.y > 1u ? info.y : 1u)) * midentity();
-    }
-    cadd(gsum, w * pg);
-    hess = hess + w * ph;
   }
+  M3 ph = system + ih;
+  if (p.objectiveFlags & 2u) {
+    M3 oh = mzero();
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const uint32_t qv = idxAt(q, l);
+      const uint4 qi = b.vinfo[qv];
+      const float kt = isPinned(qi) ? 0.0f : targetStiffness(p, b, qv) / float(qi.y > 1u ? qi.y : 1u);
+      oh = oh + kt * mm(mtrans(basis[l]), basis[l]);
+    }
+    ph = ph + oh;
+  }
+  if (ss < 4) {
+    const float3 own = ss == 0 ? tg[0] : ss == 1 ? tg[1] : ss == 2 ? tg[2] : tg[3];
+    // The inertia share is rounded before it joins the record's gradient (it
+    // belongs to the vertex, not to the record).
+    const float3 away = position - xyz(pv);
+    pg = pg - (own + f3(__fmul_rn(dWs, away.x), __fmul_rn(dWs, away.y), __fmul_rn(dWs, away.z)));
+    if (objActive) pg = pg - distributedObjective(p, b, v, position, info);
+    ph = ph - (mm(mm(R, stiffnessBlock(k, ss, ss)), mtrans(R)) + dWs * midentity());
+    if (p.objectiveFlags & 2u)
+      ph = ph - (targetStiffness(p, b, v) / float(info.y > 1u ? info.y : 1u)) * midentity();
+  }
+  pg = w * pg;
+  row[0] = pg.x; row[1] = pg.y; row[2] = pg.z;
+  row[3] = ph.c0.x; row[4] = ph.c0.y; row[5] = ph.c0.z;
+  row[6] = ph.c1.x; row[7] = ph.c1.y; row[8] = ph.c1.z;
+  row[9] = ph.c2.x; row[10] = ph.c2.y; row[11] = ph.c2.z;
+  return w;
+}
+
+__device__ __forceinline__ void storeCoRow(float* dst, const float (&row)[kCoRow]) {
+  float4* d = reinterpret_cast<float4*>(dst);
+#pragma unroll
+  for (uint32_t i = 0; i < kCoRow / 4; ++i)
+    d[i] = make_float4(row[4 * i], row[4 * i + 1], row[4 * i + 2], row[4 * i + 3]);
+}
+
+__global__ void __launch_bounds__(kBlock, 2) corotatedSolveKernel(Buffers b, const DevParams* __restrict__ pp,
+                                                               const float4* __restrict__ src, float4* tgt,
+                                                               const uint32_t* __restrict__ list, uint32_t count,
+                                                               uint32_t K) {
+  __shared__ float4 rows4[kCoVertices * kCoStride / 4];
+  __shared__ float weight[kCoVertices][kCoRecords];
+  __shared__ uint32_t sVertex[kCoVertices], sStart[kCoVertices], sCount[kCoVertices];
+  float* rows = reinterpret_cast<float*>(rows4);
+  const uint32_t first = blockIdx.x * kCoVertices;
+  uint32_t mine = 0;  // incident tets of this thread's vertex
+  if (threadIdx.x < kCoVertices) {
+    const uint32_t i = first + threadIdx.x;
+    uint32_t v = kEmptyTet;
+    if (i < count) {
+      v = list ? list[i] : i;
+      const uint4 info = b.vinfo[v];
+      if (!pp[b.vertexScene[v]].active) {
+        v = kEmptyTet;
+      } else if (isPinned(info)) {
+        const float4 rm = b.restMass[v];
+        tgt[v] = make_float4(rm.x, rm.y, rm.z, 1.0f);
+        b.finalUpdate[v] = 0.0f;
+        v = kEmptyTet;
+      } else {
+        sStart[threadIdx.x] = info.x;
+        mine = info.y;
+      }
+    }
+    sVertex[threadIdx.x] = v;
+    sCount[threadIdx.x] = mine;
+  }
+  __syncthreads();
+  uint32_t most = 0;
+  for (uint32_t g = 0; g < kCoVertices; ++g) most = max(most, sCount[g]);
+  // This thread's component sum: component `comp` (gradient 0-2, Hessian
+  // columns 3-11) of the block's vertex `sg`.
+  const uint32_t sg = threadIdx.x / kCoRow, comp = threadIdx.x % kCoRow;
+  const uint32_t sv = sg < kCoVertices ? sVertex[sg] : kEmptyTet;
+  const bool sums = sv != kEmptyTet;
+  float acc = 0.0f, low = 0.0f;  // gradient components: value and compensation
+  auto gradientAdd = [&](float x) {
+    float e;
+    acc = twoSum(acc, x, &e);
+    low = __fadd_rn(low, e);
+  };
+  auto component = [&](float3 a) { return comp == 0 ? a.x : comp == 1 ? a.y : a.z; };
+  const bool diagonal = comp == 3 || comp == 7 || comp == 11;
+  if (sums) {
+    const DevParams& p = pp[b.vertexScene[sv]];
+    const float4 rm = b.restMass[sv];
+    const float inertia = rm.w * p.invDt2;
+    if (comp < 3) {
+      const float3 position = xyz(src[sv]);
+      gradientAdd(component(inertia * (position - xyz(b.predicted[sv]))));
+      if (p.objectiveFlags != 0u) gradientAdd(component(objectiveGradient(p, b, sv, position)));
+    } else if (diagonal) {
+      acc = inertia;
+      if (p.objectiveFlags & 2u) acc = __fadd_rn(acc, targetStiffness(p, b, sv));
+    }
+  }
+  auto record = [&](uint32_t g, uint32_t j, uint32_t s0) {
+    const uint32_t v = sVertex[g];
+    if (v == kEmptyTet) return;
+    float row[kCoRow];
+    const float w = corotatedRecord(b, pp[b.vertexScene[v]], src, v, static_cast<size_t>(v) * K + s0 + j, row);
+    weight[g][j] = w;
+    if (w > 0.0f) storeCoRow(rows + g * kCoStride + (kCoTets + j) * kCoRow, row);
+  };
+  auto tet = [&](uint32_t g, uint32_t j, uint32_t a0) {
+    if (a0 + j >= sCount[g]) return;
+    const uint32_t entry = __ldg(&b.adjacency[sStart[g] + a0 + j]);
+    const uint32_t t = entry >> 2, slot = entry & 3u;
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(b.tets) + 4ull * t + 3);
+    const M3 R = loadRot(b.tetRot, t);
+    const float* k = b.stiffness + 144ull * t;
+    float3 disp[4];
+    corotatedDisplacement(b, src, q, R, disp);
+    const float3 tg = stiffnessTimes(stiffnessRow(k, slot), R, disp);
+    const M3 h = mm(mm(R, stiffnessBlock(k, slot, slot)), mtrans(R));
+    const float row[kCoRow] = {tg.x, tg.y, tg.z, h.c0.x, h.c0.y, h.c0.z, h.c1.x, h.c1.y, h.c1.z, h.c2.x, h.c2.y, h.c2.z};
+    storeCoRow(rows + g * kCoStride + j * kCoRow, row);
+  };
+  // The first records (the long items) go first and beside the first tets;
+  // their rows wait until the tets are added.
+  const uint32_t firstRecords = min(kCoRecords, K);
+  for (uint32_t item = threadIdx.x; item < kCoVertices * (firstRecords + kCoTets); item += kBlock) {
+    if (item < kCoVertices * firstRecords) {
+      record(item / firstRecords, item % firstRecords, 0);
+    } else {
+      const uint32_t i = item - kCoVertices * firstRecords;
+      tet(i / kCoTets, i % kCoTets, 0);
+    }
+  }
+  for (uint32_t a0 = 0; a0 == 0 || a0 < most; a0 += kCoTets) {
+    if (a0 > 0)
+      for (uint32_t item = threadIdx.x; item < kCoVertices * kCoTets; item += kBlock)
+        tet(item / kCoTets, item % kCoTets, a0);
+    __syncthreads();
+    if (sums) {
+      const uint32_t n = min(kCoTets, sCount[sg] > a0 ? sCount[sg] - a0 : 0u);
+      const float* r = rows + sg * kCoStride + comp;
+      if (comp < 3)
+        for (uint32_t j = 0; j < n; ++j) gradientAdd(r[j * kCoRow]);
+      else
+        for (uint32_t j = 0; j < n; ++j) acc = __fadd_rn(acc, r[j * kCoRow]);
+    }
+    __syncthreads();
+  }
+  if (sums && (comp == 1 || comp == 7)) {
+    const DevParams& p = pp[b.vertexScene[sv]];
+    const float y = src[sv].y;
+    if (p.floorStiffness > 0.0f && y < p.floorHeight) {
+      if (comp == 1) gradientAdd(p.floorStiffness * (y - p.floorHeight));
+      else acc = __fadd_rn(acc, p.floorStiffness);
+    }
+  }
+  for (uint32_t s0 = 0; s0 < K; s0 += kCoRecords) {
+    const uint32_t n = min(kCoRecords, K - s0);
+    if (s0 > 0) {
+      __syncthreads();
+      for (uint32_t item = threadIdx.x; item < kCoVertices * n; item += kBlock) record(item / n, item % n, s0);
+      __syncthreads();
+    }
+    if (sums) {
+      const float* r = rows + sg * kCoStride + kCoTets * kCoRow + comp;
+      for (uint32_t j = 0; j < n; ++j) {
+        const float w = weight[sg][j];
+        if (!(w > 0.0f)) continue;
+        if (comp < 3) gradientAdd(r[j * kCoRow]);
+        else acc = __fmaf_rn(w, r[j * kCoRow], acc);
+      }
+    }
+  }
+  if (sums) rows[sg * kCoStride + comp] = comp < 3 ? __fadd_rn(acc, low) : acc;
+  __syncthreads();
+  if (threadIdx.x >= kCoVertices || sVertex[threadIdx.x] == kEmptyTet) return;
+  const uint32_t v = sVertex[threadIdx.x];
+  const DevParams& p = pp[b.vertexScene[v]];
+  const float* r = rows + threadIdx.x * kCoStride;
+  const float3 gradient = f3(r[0], r[1], r[2]);
+  const M3 hess = {f3(r[3], r[4], r[5]), f3(r[6], r[7], r[8]), f3(r[9], r[10], r[11])};
+  const float3 position = xyz(src[v]);
   // Regularised Cholesky solve with the shift max(regularization * scale, 1e-9).
   const float ds = fmaxf(1.0f, fmaxf(fabsf(hess.c0.x), fmaxf(fabsf(hess.c1.y), fabsf(hess.c2.z))));
   const float shift = fmaxf(p.regularization * ds, 1.0e-9f);
@@ -814,7 +1013,7 @@ __global__ void __launch_bounds__(kBlock) corotatedSolveKernel(Buffers b, const 
   const float a01 = 0.5f * (hess.c0.y + hess.c1.x);
   const float a02 = 0.5f * (hess.c0.z + hess.c2.x);
   const float a12 = 0.5f * (hess.c1.z + hess.c2.y);
-  const float3 rhs = -cvalue(gsum);
+  const float3 rhs = -gradient;
   const float l00 = sqrtf(fmaxf(a00, shift));
   const float l10 = a01 / l00, l20 = a02 / l00;
   const float l11 = sqrtf(fmaxf(a11 - l10 * l10, shift));
@@ -823,13 +1022,15 @@ __global__ void __launch_bounds__(kBlock) corotatedSolveKernel(Buffers b, const 
   const float y0 = rhs.x / l00, y1 = (rhs.y - l10 * y0) / l11, y2 = (rhs.z - l20 * y0 - l21 * y1) / l22;
   const float x2 = y2 / l22, x1 = (y1 - l21 * x2) / l11, x0 = (y0 - l10 * x1 - l20 * x2) / l00;
   float3 delta = f3(x0, x1, x2);
-  const float sq = dot3(delta, delta);
+  // The fused form every step bound and update record has been taken with.
+  auto squared = [](float3 d) { return __fmaf_rn(d.z, d.z, __fmaf_rn(d.x, d.x, __fmul_rn(d.y, d.y))); };
+  const float sq = squared(delta);
   if (!(sq >= 0.0f && sq < 1.0e30f)) delta = f3(0, 0, 0);
-  const float dls = dot3(delta, delta);
+  const float dls = squared(delta);
   if (p.maxStep > 0.0f && dls > p.maxStep * p.maxStep) delta = delta * (p.maxStep * (1.0f / sqrtf(dls)));
   const float3 np = position + delta;
   tgt[v] = make_float4(np.x, np.y, np.z, 1.0f);
-  b.finalUpdate[v] = sqrtf(dot3(delta, delta));
+  b.finalUpdate[v] = sqrtf(squared(delta));
 }
 
 __global__ void __launch_bounds__(kBlock) copyKernel(Buffers b, const DevParams* __restrict__ pp,
@@ -3578,14 +3779,16 @@ int launchTetPolar(const Buffers& b, const DevParams* p, const float4* src, uint
 int launchCorotatedSolve(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
                          uint32_t count, uint32_t K, cudaStream_t s) {
   if (count == 0) return 0;
-  corotatedSolveKernel<<<blocksFor(count), kBlock, 0, s>>>(b, p, src, tgt, list, count, K);
+  corotatedSolveKernel<<<(count + kCoVertices - 1) / kCoVertices, kBlock, 0, s>>>(b, p, src, tgt, list, count, K);
   return 1;
 }
 
 int launchVertexPolar(const Buffers& b, const DevParams* p, const float4* src, const uint32_t* list,
                       uint32_t count, cudaStream_t s) {
   if (count == 0) return 0;
-  vertexPolarKernel<<<blocksFor(count), kBlock, 0, s>>>(b, p, src, list, count);
+  if (count <= kWideVertices)
+    vertexPolarKernel<true><<<(count + kConvChunk - 1) / kConvChunk, kWideBlock, 0, s>>>(b, p, src, list, count);
+  else vertexPolarKernel<false><<<blocksFor(count), kBlock, 0, s>>>(b, p, src, list, count);
   return 1;
 }
 
