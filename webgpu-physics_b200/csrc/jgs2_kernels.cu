@@ -68,15 +68,22 @@ __device__ __forceinline__ bool tetVerticesInBounds(const uint4& q, uint32_t V) 
 // Lanes per vertex in the solve kernel.  A warp holds 32 / kGroup lane groups;
 // a width that does not divide 32 leaves the warp's last lanes idle.
 constexpr int kGroup = JGS2_SOLVE_LANES;
-#ifndef JGS2_FRAME_QUAT
-#define JGS2_FRAME_QUAT 0
-#endif
 // Incident-tet gathers request the next tet's record before the current
 // one's arithmetic (convergence, frames, the line search).
 #ifndef JGS2_CONV_LOOKAHEAD
 #define JGS2_CONV_LOOKAHEAD 1
 #endif
 constexpr int kRecFloats = 56;  // cached cubature record state
+
+// Two float4 by one 256-bit load of data no kernel in flight writes, from a
+// 32-byte boundary.  A gather's cost is its cache-line lookups, one per lane
+// and instruction, not its bytes: a 64-byte record by two such loads takes
+// half the lookups of four 128-bit ones.
+__device__ __forceinline__ void load256(const float4* __restrict__ p, float4& a, float4& b) {
+  asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
 
 struct TetRec {
   float3 g1, g2, g3;
@@ -85,10 +92,10 @@ struct TetRec {
 };
 
 __device__ __forceinline__ TetRec loadTet(const float4* __restrict__ tets, uint32_t t) {
-  const float4 a = __ldg(&tets[4ull * t]);
-  const float4 b = __ldg(&tets[4ull * t + 1]);
-  const float4 c = __ldg(&tets[4ull * t + 2]);
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(tets) + 4ull * t + 3);
+  float4 a, b, c, d;
+  load256(tets + 4ull * t, a, b);
+  load256(tets + 4ull * t + 2, c, d);
+  const uint4 q = make_uint4(__float_as_uint(d.x), __float_as_uint(d.y), __float_as_uint(d.z), __float_as_uint(d.w));
   TetRec r;
   r.g1 = f3(a.x, a.y, a.z);
   r.g2 = f3(b.x, b.y, b.z);
@@ -145,17 +152,14 @@ __device__ __forceinline__ float4 ldPos(const float4* p, size_t i) {
   if constexpr (kCoherent) return __ldca(p + i);
   else return p[i];
 }
-__device__ __forceinline__ M3 quaternionFrame(float4 q);
 template <bool kCoherent>
-__device__ __forceinline__ M3 loadRotT(const float4* rot, uint32_t v) {
-#if JGS2_FRAME_QUAT
-  return quaternionFrame(kCoherent ? __ldca(rot + 3ull * v) : rot[3ull * v]);
-#endif
+__device__ __forceinline__ M3 loadFrameT(const float4* pack, uint32_t v) {
   if constexpr (kCoherent) {
-    const float4 a = __ldca(rot + 3ull * v), b = __ldca(rot + 3ull * v + 1), c = __ldca(rot + 3ull * v + 2);
+    const float4 a = __ldca(pack + 4ull * v), b = __ldca(pack + 4ull * v + 1), c = __ldca(pack + 4ull * v + 2);
     return {f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), f3(c.x, c.y, c.z)};
   } else {
-    return loadRot(rot, v);
+    const float4 a = pack[4ull * v], b = pack[4ull * v + 1], c = pack[4ull * v + 2];
+    return {f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), f3(c.x, c.y, c.z)};
   }
 }
 template <bool kCoherent>
@@ -173,52 +177,29 @@ __device__ __forceinline__ void storeRot(float4* __restrict__ rot, uint32_t v, c
   rot[3ull * v + 2] = make_float4(m.c2.x, m.c2.y, m.c2.z, 0.f);
 }
 
-// Vertex frames.  With JGS2_FRAME_QUAT a frame is stored as a unit
-// quaternion in the first float4 of its three (one vector load per read
-// instead of three); the matrix is rebuilt from it on every read.
-__device__ __forceinline__ float4 frameQuaternion(const M3& m) {
-  // Shepperd's method on the largest of the trace and the diagonal.
-  const float m00 = m.c0.x, m11 = m.c1.y, m22 = m.c2.z;
-  const float m21 = m.c1.z, m12 = m.c2.y, m02 = m.c2.x, m20 = m.c0.z, m10 = m.c0.y, m01 = m.c1.x;
-  const float tr = m00 + m11 + m22;
-  float4 q;
-  if (tr > 0.0f) {
-    const float t = sqrtf(tr + 1.0f) * 2.0f;
-    q = make_float4((m21 - m12) / t, (m02 - m20) / t, (m10 - m01) / t, 0.25f * t);
-  } else if (m00 > m11 && m00 > m22) {
-    const float t = sqrtf(1.0f + m00 - m11 - m22) * 2.0f;
-    q = make_float4(0.25f * t, (m01 + m10) / t, (m02 + m20) / t, (m21 - m12) / t);
-  } else if (m11 > m22) {
-    const float t = sqrtf(1.0f + m11 - m00 - m22) * 2.0f;
-    q = make_float4((m01 + m10) / t, 0.25f * t, (m12 + m21) / t, (m02 - m20) / t);
-  } else {
-    const float t = sqrtf(1.0f + m22 - m00 - m11) * 2.0f;
-    q = make_float4((m02 + m20) / t, (m12 + m21) / t, 0.25f * t, (m10 - m01) / t);
-  }
-  const float n = rsqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
-  return make_float4(q.x * n, q.y * n, q.z * n, q.w * n);
+// The frame of vertex v and its position at the same pose into the vertex's
+// pack (its inertial target is the prologue's).
+__device__ __forceinline__ void storeFrame(float4* __restrict__ pack, uint32_t v, const M3& m, float3 x) {
+  pack[4ull * v] = make_float4(m.c0.x, m.c0.y, m.c0.z, x.x);
+  pack[4ull * v + 1] = make_float4(m.c1.x, m.c1.y, m.c1.z, x.y);
+  pack[4ull * v + 2] = make_float4(m.c2.x, m.c2.y, m.c2.z, x.z);
 }
-__device__ __forceinline__ M3 quaternionFrame(float4 q) {
-  const float x2 = q.x + q.x, y2 = q.y + q.y, z2 = q.z + q.z;
-  const float xx = q.x * x2, yy = q.y * y2, zz = q.z * z2;
-  const float xy = q.x * y2, xz = q.x * z2, yz = q.y * z2;
-  const float wx = q.w * x2, wy = q.w * y2, wz = q.w * z2;
-  return {f3(1.0f - (yy + zz), xy + wz, xz - wy), f3(xy - wz, 1.0f - (xx + zz), yz + wx),
-          f3(xz + wy, yz - wx, 1.0f - (xx + yy))};
+__device__ __forceinline__ M3 loadFrame(const float4* __restrict__ pack, uint32_t v) {
+  return loadFrameT<false>(pack, v);
 }
-__device__ __forceinline__ void storeFrame(float4* __restrict__ rot, uint32_t v, const M3& m) {
-#if JGS2_FRAME_QUAT
-  rot[3ull * v] = frameQuaternion(m);
-#else
-  storeRot(rot, v, m);
-#endif
-}
-__device__ __forceinline__ M3 loadFrame(const float4* __restrict__ rot, uint32_t v) {
-#if JGS2_FRAME_QUAT
-  return quaternionFrame(rot[3ull * v]);
-#else
-  return loadRot(rot, v);
-#endif
+
+// What a record's tet needs of one of its vertices: frame, source position,
+// inertial target and distributed inertia weight, 64 bytes in one place.
+struct VertexPack {
+  M3 R;
+  float3 x, pred;
+  float dW;
+};
+__device__ __forceinline__ VertexPack loadPack(const float4* __restrict__ pack, uint32_t v) {
+  float4 a, b, c, d;
+  load256(pack + 4ull * v, a, b);
+  load256(pack + 4ull * v + 2, c, d);
+  return {{xyz(a), xyz(b), xyz(c)}, f3(a.w, b.w, c.w), xyz(d), d.w};
 }
 
 // Row-major stored Ubar block l -> columns (cubatureBlock, jgs2-shader.ts:1204-1212).
@@ -589,7 +570,7 @@ __device__ __forceinline__ void storeFrameAndIncident(const Buffers& b, const De
     clothLocalSystem<true>(b.clothTris, b.clothHinges, b.clothIncidence, b.clothRange[v], x, clothMaterial(p), 0u, 1u,
                            o.grad, o.hess);
   const M3 favg = o.total > 0.0f ? (1.0f / o.total) * o.avg : midentity();
-  storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
+  storeFrame(b.vertexPack, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon), xyz(x[v]));
   storeIncident(b.incident, v, cvalue(o.grad), o.hess);
 }
 
@@ -639,8 +620,9 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) vertexPolarKernel
     if (threadIdx.x < kConvChunk && wanted(first + threadIdx.x, &v)) {
       const IncidentSums sums = loadIncidentSums(sh.sums[threadIdx.x]);
       const M3 avg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
-      storeFrame(b.vertexRot, v,
-                 b.vinfo[v].y == 0u ? midentity() : polarRotation(avg, pp[b.vertexScene[v]].rotationEpsilon));
+      storeFrame(b.vertexPack, v,
+                 b.vinfo[v].y == 0u ? midentity() : polarRotation(avg, pp[b.vertexScene[v]].rotationEpsilon),
+                 xyz(x[v]));
     }
   } else {
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
@@ -649,7 +631,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) vertexPolarKernel
     const uint32_t scene = b.vertexScene[v];
     const DevParams& p = pp[scene];
     if (!p.active || latched(p, &b.frames[scene])) return;
-    storeFrame(b.vertexRot, v, vertexFrame(b, x, v, p.rotationEpsilon));
+    storeFrame(b.vertexPack, v, vertexFrame(b, x, v, p.rotationEpsilon), xyz(x[v]));
   }
 }
 
@@ -769,14 +751,14 @@ __device__ __forceinline__ float3 distributedObjective(const DevParams& p, const
 // and Hessian (9) contribution goes to shared memory, then 12 threads per
 // vertex add one component each over the items in order (the vertex's own
 // terms, incident tets in adjacency order, floor, records in record order),
-// and one thread per vertex solves.  One thread per vertex for all of it, as
-// before, ran a chain of 24 tets and K records of 144-float stiffness
-// matrices serially: 322 us per launch at 1 200 vertices whatever the GPU had
-// idle.  The contributions and the order of the sums are the same, so are the
-// bits.
-#ifndef JGS2_CO_MIN_BLOCKS
-#define JGS2_CO_MIN_BLOCKS 2
-#endif
+// and one thread per vertex solves.  Bound by the latency of an item's gathers
+// and its 144-float stiffness, of which every float is loaded once, nine
+// vector loads a block row.  One thread per vertex for all of it, as before,
+// walked 24 tets and K records one after another and loaded the stiffness
+// four times: 322 us per launch at 1 200 vertices (now 17), 340 at 9 020 (now
+// 49).  The contributions and the order of the sums are the same, so are the
+// bits.  Two blocks per SM (246 registers, no spills); three spill 220 bytes,
+// gain 6 % at 9 020 vertices and lose 3 % at 1 200.
 constexpr uint32_t kCoVertices = 10;   // 120 component sums on 128 threads
 constexpr uint32_t kCoTets = 24;       // incident tets of a vertex per round
 constexpr uint32_t kCoRecords = 8;     // records of a vertex per round
@@ -795,13 +777,13 @@ __device__ __forceinline__ float corotatedRecord(const Buffers& b, const DevPara
   const float4 pv = b.predicted[v];
   const float dWs = pv.w;
   const bool objActive = p.objectiveFlags != 0u;
-  const M3 RsT = mtrans(loadFrame(b.vertexRot, v));
+  const M3 RsT = mtrans(loadFrame(b.vertexPack, v));
   const uint32_t t = head.x;
   const uint4 q = __ldg(&b.cubHead[2 * rec + 1]);
   const float4* U = b.cubBasis + 9ull * rec;
   M3 basis[4];
 #pragma unroll
-  for (int l = 0; l < 4; ++l) basis[l] = mm(mm(loadFrame(b.vertexRot, idxAt(q, l)), loadBlockVec(U, l)), RsT);
+  for (int l = 0; l < 4; ++l) basis[l] = mm(mm(loadFrame(b.vertexPack, idxAt(q, l)), loadBlockVec(U, l)), RsT);
   const M3 R = loadRot(b.tetRot, t);
   const float* k = b.stiffness + 144ull * t;
   float3 disp[4], tg[4];
@@ -2130,6 +2112,59 @@ __device__ __forceinline__ M3 loadBlockVecShared(const float4* rec, int l) {
 // the tet's material and, when v is one of the tet's vertices, its slot and
 // shape gradient.  Read from the block's staged slot or from global memory;
 // st.w = 0 for an empty record.  `r` receives the record's tet.
+template <bool kCoherent, class Basis>
+__device__ __forceinline__ void recordStateOf(const Buffers& b, const DevParams& p, uint32_t v, float w, const uint4& idx,
+                                              const TetRec& r, Basis basis, const float4* __restrict__ src,
+                                              bool objActive, CubState& st) {
+  M3 F = mzero(), dF0 = mzero(), dF1 = mzero(), dF2 = mzero();
+  float3 gQ = f3(0, 0, 0);
+  S3 HQ = szero();
+  uint32_t slot = 4;
+  float3 x0 = f3(0, 0, 0);
+#pragma unroll
+  for (int l = 0; l < 4; ++l) {
+    const uint32_t q = idxAt(idx, l);
+    if (q == v) slot = l;
+    const float3 gl = shapeGradient(r, l);
+    VertexPack pk;
+    if constexpr (kCoherent) {
+      const float4 pq = b.predicted[q];
+      pk = {loadFrameT<true>(b.vertexPack, q), xyz(__ldca(src + q)), xyz(pq), pq.w};
+    } else {
+      pk = loadPack(b.vertexPack, q);
+    }
+    const M3 B = mm(pk.R, basis(l));
+    const float3 xl = pk.x;
+    if (l == 0) x0 = xl;
+    if (l > 0) F = F + outer(xl - x0, gl);
+    dF0 = dF0 + outer(B.c0, gl);
+    dF1 = dF1 + outer(B.c1, gl);
+    dF2 = dF2 + outer(B.c2, gl);
+    // The distributed inertia weight is 0 when pinned.
+    const float dW = pk.dW;
+    float3 lin = dW * (xl - pk.pred);
+    float quad = dW;
+    const uint4 qi = objActive ? b.vinfo[q] : make_uint4(0u, 0u, 1u, 0u);
+    if (objActive && !isPinned(qi)) {
+      const float nq = float(qi.y > 1u ? qi.y : 1u);
+      lin = lin + objectiveGradient(p, b, q, xl) * (1.0f / nq);
+      quad += targetStiffness(p, b, q) / nq;
+    }
+    gQ = gQ + mtv(B, lin);
+    saddScaled(HQ, quad, gramColumns(B));
+  }
+  st.F = F;
+  st.I0 = frob(F, F);
+  st.J0 = mdet(F);
+  st.dF0 = dF0; st.dF1 = dF1; st.dF2 = dF2;
+  st.gQ = gQ;
+  st.HQ = HQ;
+  st.w = w;
+  st.vol = r.vol; st.lambda = r.lambda; st.mu = r.mu;
+  st.slot = slot;
+  st.gs = slot < 4 ? shapeGradient(r, slot) : f3(0, 0, 0);
+}
+
 template <bool kCoherent, bool kStaged>
 __device__ __forceinline__ void recordState(const Buffers& b, const DevParams& p, uint32_t v, size_t rec,
                                             const RecSlot* staged, const float4* __restrict__ src, bool objActive,
@@ -2151,56 +2186,15 @@ __device__ __forceinline__ void recordState(const Buffers& b, const DevParams& p
       !inBounds(idx.y, b.vertexTotal, kSiteRecordVertex) || !inBounds(idx.z, b.vertexTotal, kSiteRecordVertex) ||
       !inBounds(idx.w, b.vertexTotal, kSiteRecordVertex))
     return;
-  const float4* U;
   if constexpr (kStaged) {
     r = tetFromSlot(staged->tet);
-    U = staged->basis;
+    recordStateOf<kCoherent>(b, p, v, w, idx, r, [&](int l) { return loadBlockVecShared(staged->basis, l); }, src,
+                             objActive, st);
   } else {
     r = loadTet(b.tets, t);
-    U = b.cubBasis + 9ull * rec;
+    const float4* U = b.cubBasis + 9ull * rec;
+    recordStateOf<kCoherent>(b, p, v, w, idx, r, [&](int l) { return loadBlockVec(U, l); }, src, objActive, st);
   }
-  M3 F = mzero(), dF0 = mzero(), dF1 = mzero(), dF2 = mzero();
-  float3 gQ = f3(0, 0, 0);
-  S3 HQ = szero();
-  uint32_t slot = 4;
-  const float3 x0 = xyz(ldPos<kCoherent>(src, idx.x));
-#pragma unroll
-  for (int l = 0; l < 4; ++l) {
-    const uint32_t q = idxAt(idx, l);
-    if (q == v) slot = l;
-    const float3 gl = shapeGradient(r, l);
-    M3 B;
-    if constexpr (kStaged) B = mm(loadRotT<kCoherent>(b.vertexRot, q), loadBlockVecShared(U, l));
-    else B = mm(loadRotT<kCoherent>(b.vertexRot, q), loadBlockVec(U, l));
-    const float3 xl = l == 0 ? x0 : xyz(ldPos<kCoherent>(src, q));
-    if (l > 0) F = F + outer(xl - x0, gl);
-    dF0 = dF0 + outer(B.c0, gl);
-    dF1 = dF1 + outer(B.c1, gl);
-    dF2 = dF2 + outer(B.c2, gl);
-    // predicted w = distributed inertia weight (0 when pinned).
-    const float4 pq = b.predicted[q];
-    const float dW = pq.w;
-    float3 lin = dW * (xl - xyz(pq));
-    float quad = dW;
-    const uint4 qi = objActive ? b.vinfo[q] : make_uint4(0u, 0u, 1u, 0u);
-    if (objActive && !isPinned(qi)) {
-      const float nq = float(qi.y > 1u ? qi.y : 1u);
-      lin = lin + objectiveGradient(p, b, q, xl) * (1.0f / nq);
-      quad += targetStiffness(p, b, q) / nq;
-    }
-    gQ = gQ + mtv(B, lin);
-    saddScaled(HQ, quad, gramColumns(B));
-  }
-  st.F = F;
-  st.I0 = frob(F, F);
-  st.J0 = mdet(F);
-  st.dF0 = dF0; st.dF1 = dF1; st.dF2 = dF2;
-  st.gQ = gQ;
-  st.HQ = HQ;
-  st.w = w;
-  st.vol = r.vol; st.lambda = r.lambda; st.mu = r.mu;
-  st.slot = slot;
-  st.gs = slot < 4 ? shapeGradient(r, slot) : f3(0, 0, 0);
 }
 
 // One block's chunk `chunk` of the vertex list: vertices
@@ -2320,7 +2314,7 @@ __device__ __forceinline__ void solveChunk(const Buffers& b, const DevParams* __
         // B'_l = R_l Ubar_l, so R_s is applied once per record instead of once
         // per basis block.  The exact source block subtracted for a record at
         // the vertex's own slot is formed in the world frame.
-        const M3 Rs = loadRotT<kCoherent>(b.vertexRot, v);
+        const M3 Rs = loadFrameT<kCoherent>(b.vertexPack, v);
         unsigned char* mySlots = slotBase + static_cast<size_t>(group) * K * kSolveSlotBytes;
         // Cubature records first, then (unless cached) the incident tets, in
         // separate loops so the two kinds of item never share a divergent pass.
@@ -2701,6 +2695,747 @@ __global__ void __launch_bounds__(kBlock, JGS2_SOLVE_MIN_BLOCKS) solveKernel(Buf
 }
 
 // ---------------------------------------------------------------------------
+// The same local solve with the block's work spread over its threads by item
+// instead of by vertex: solid scenes (no cloth, no contact) whose records fit
+// shared memory.  A block takes up to kG vertices and goes through
+//   records   one thread per cubature record: its state to shared memory, its
+//             gradient and Hessian contribution to a row;
+//   incident  (coloured sweeps) one thread per incident tet, likewise;
+//   sums      four lanes per vertex add the rows in solveChunk's order;
+//   solve     one thread per vertex: globalization and the line search's
+//             bookkeeping;
+//   trial     per line-search trial one thread per record and per incident tet
+//             evaluates its energy delta and determinant, and four lanes per
+//             vertex add them.
+// A record's or tet's arithmetic and the order of every sum are solveChunk's,
+// so a vertex takes the same step, bit for bit, in either kernel and for any
+// kG (the recorded energy delta of an accepted trial can differ in its last
+// bit).
+//
+// Bound by latency: with few vertices a launch is one block's chain of
+// phases.  solveChunk's chain is two passes of four lanes over six records,
+// six passes over 24 incident tets per trial and up to 13 trials; here a
+// record or tet is one pass and, at eight vertices a block, a thread keeps its
+// incident tet's deformation gradient over the trials and four backtracked
+// trials are evaluated at a time.  Measured per launch (events; four lanes,
+// then items): 525 vertices 27.0 / 18.9 us, 2 688 vertices 35 / 27, 13 392
+// vertices 44.6 / 39.4; one colour of the 525-vertex bar, whose trials a
+// determinant bound often holds back, 72 / 33, of a 27 360-vertex block
+// 85 / 36.  A large solve is better off with four lanes (1 030 301 vertices:
+// 1.72 ms, 1.79 by items, 68 921: 139 / 142 us): both run out of warps to hide
+// the gathers behind, and the block's barriers then cost more than the idle
+// lanes.
+constexpr uint32_t kItemTrials = 4;   // backtracked trials evaluated at a time
+constexpr uint32_t kItemTets = 24;    // incident tets of a vertex per round (the grid meshes' largest valence)
+constexpr uint32_t kBasisWords = 9;   // float4 per record: basis blocks, then dF (27), gQ (3), HQ (6)
+constexpr uint32_t kStateWords = 5;   // float4 per record: F, vol, lambda, mu, gs, w, I0, J0, slot; an odd stride
+constexpr uint32_t kRowFloats = 18;   // floats per record row: w R_s g (3), R_s H R_s^T (6), own block (3 + 6)
+constexpr uint32_t kTetRowFloats = 10;  // floats per incident row: gradient (3), Hessian block (6), vol
+
+__host__ __device__ constexpr uint32_t itemScratchFloats(uint32_t groups, uint32_t K, bool incident, uint32_t trials) {
+  const uint32_t gather = groups * (K * kRowFloats + (incident ? kItemTets * kTetRowFloats : 0u));
+  const uint32_t trial = trials * groups * (K * 2u + kItemTets * 3u);
+  return ((gather > trial ? gather : trial) + 3u) & ~3u;
+}
+__host__ __device__ constexpr size_t itemSharedBytes(uint32_t groups, uint32_t K, bool incident, uint32_t trials) {
+  return size_t(groups) * K * (kBasisWords + kStateWords) * 16 +
+         size_t(itemScratchFloats(groups, K, incident, trials)) * 4;
+}
+
+template <uint32_t kG, uint32_t kT>
+struct ItemShared {
+  uint32_t v[kG], scene[kG], start[kG], count[kG];
+  uint32_t solve[kG];            // the vertex takes a local solve
+  uint32_t eval[kG];             // trials of it to evaluate this round
+  // Per trial of the round: the step, the step in the vertex's frame and the
+  // terms a record at the vertex's own slot takes out.
+  float td[kT][kG][3], ts[kT][kG][3], ownMove[kT][kG], ownObjective[kT][kG];
+  float sum[kG][12];             // gradient, its compensation, Hessian
+  float4 own[kG][6];             // staged: source pose, target, rest and mass, incident system
+  float de[kT][kG], jmin[kT][kG];
+  uint32_t finite[kT][kG];
+  uint32_t fail, maxBack, skip, evals, maxShift, valid;
+};
+
+// An incident tet's terms with every fused multiply-add spelled out (the first
+// product fused onto the second, as the compiler contracts the plain
+// expressions of solveChunk): the coloured sweep amplifies a last bit to whole
+// steps, and the compiler contracts differently once the deformation gradient
+// is kept across phases.
+namespace fused {
+__device__ __forceinline__ float sum2(float a, float x, float b, float y) { return __fmaf_rn(a, x, __fmul_rn(b, y)); }
+__device__ __forceinline__ float diff2(float a, float x, float b, float y) { return __fmaf_rn(a, x, -__fmul_rn(b, y)); }
+__device__ __forceinline__ float dot(float3 a, float3 b) { return __fmaf_rn(a.z, b.z, sum2(a.x, b.x, a.y, b.y)); }
+__device__ __forceinline__ float3 cross(float3 a, float3 b) {
+  return f3(diff2(a.y, b.z, a.z, b.y), diff2(a.z, b.x, a.x, b.z), diff2(a.x, b.y, a.y, b.x));
+}
+// a x + b y + c z, column by column.
+__device__ __forceinline__ float3 combine(float3 a, float x, float3 b, float y, float3 c, float z) {
+  return f3(__fmaf_rn(c.x, z, sum2(a.x, x, b.x, y)), __fmaf_rn(c.y, z, sum2(a.y, x, b.y, y)),
+            __fmaf_rn(c.z, z, sum2(a.z, x, b.z, y)));
+}
+__device__ __forceinline__ float3 timesF(const M3& m, float3 v) { return combine(m.c0, v.x, m.c1, v.y, m.c2, v.z); }
+__device__ __forceinline__ M3 cofactorF(const M3& f) { return {cross(f.c1, f.c2), cross(f.c2, f.c0), cross(f.c0, f.c1)}; }
+__device__ __forceinline__ float det(const M3& f) { return dot(f.c0, cross(f.c1, f.c2)); }
+__device__ __forceinline__ float squared(const M3& f) {
+  return __fadd_rn(__fadd_rn(dot(f.c0, f.c0), dot(f.c1, f.c1)), dot(f.c2, f.c2));
+}
+__device__ __forceinline__ M3 deformation(const TetRec& r, const float4* __restrict__ x) {
+  const float3 o = xyz(x[r.idx.x]);
+  const float3 a = xyz(x[r.idx.y]) - o, b = xyz(x[r.idx.z]) - o, c = xyz(x[r.idx.w]) - o;
+  return {combine(a, r.g1.x, b, r.g2.x, c, r.g3.x), combine(a, r.g1.y, b, r.g2.y, c, r.g3.y),
+          combine(a, r.g1.z, b, r.g2.z, c, r.g3.z)};
+}
+
+// Gradient vol P g and Hessian block (without vol) of the tet's vertex with
+// shape gradient g (piolaTerms, piola, incidentBlock).
+__device__ __forceinline__ void incident(const M3& F, float3 g, float vol, float lambda, float mu, float3* grad,
+                                         S3* block) {
+  const float den = squared(F) + 1.0f;
+  const M3 cof = cofactorF(F);
+  const float J = dot(F.c0, cof.c0);
+  const float a = __fmul_rn(mu, 1.0f - 1.0f / den);
+  const float b = diff2(lambda, J - 1.0f, 0.75f, mu);
+  const float c1 = __fmul_rn(2.0f, mu) / __fmul_rn(den, den);
+  auto stress = [&](float3 f, float3 c) { return f3(sum2(a, f.x, b, c.x), sum2(a, f.y, b, c.y), sum2(a, f.z, b, c.z)); };
+  const M3 P = {stress(F.c0, cof.c0), stress(F.c1, cof.c1), stress(F.c2, cof.c2)};
+  const float3 Pg = timesF(P, g), u = timesF(F, g), w = timesF(cof, g);
+  *grad = f3(__fmul_rn(vol, Pg.x), __fmul_rn(vol, Pg.y), __fmul_rn(vol, Pg.z));
+  const float d = __fmul_rn(a, dot(g, g));
+  auto entry = [&](float diagonal, float u0, float u1, float w0, float w1) {
+    return __fmaf_rn(__fmul_rn(lambda, w0), w1, __fmaf_rn(__fmul_rn(c1, u0), u1, diagonal));
+  };
+  *block = {entry(d, u.x, u.x, w.x, w.x),    entry(d, u.y, u.y, w.y, w.y),    entry(d, u.z, u.z, w.z, w.z),
+            entry(0.0f, u.x, u.y, w.x, w.y), entry(0.0f, u.x, u.z, w.x, w.z), entry(0.0f, u.y, u.z, w.y, w.z)};
+}
+
+// snhEnergyDeltaRankOne of a step d of that vertex.
+__device__ __forceinline__ float energyDelta(const M3& F, float3 d, float3 g, float lambda, float mu, float* Jtrial) {
+  const float I0 = squared(F), J0 = det(F);
+  const float id = __fmaf_rn(dot(d, d), dot(g, g), __fmul_rn(2.0f, dot(d, timesF(F, g))));
+  const float dj = dot(d, timesF(cofactorF(F), g));
+  auto moved = [&](float3 c, float s) { return f3(__fmaf_rn(d.x, s, c.x), __fmaf_rn(d.y, s, c.y), __fmaf_rn(d.z, s, c.z)); };
+  const M3 f1 = {moved(F.c0, g.x), moved(F.c1, g.y), moved(F.c2, g.z)};
+  const float J1 = det(f1);
+  *Jtrial = J1;
+  const float lr = logOnePlus(id / (I0 + 1.0f));
+  const float half = __fmul_rn(0.5f, mu);
+  float e = diff2(half, id, __fmul_rn(0.75f, mu), dj);
+  e = __fmaf_rn(__fmul_rn(__fmul_rn(0.5f, lambda), dj), J1 + J0 - 2.0f, e);
+  return __fmaf_rn(-half, lr, e);
+}
+}  // namespace fused
+
+template <uint32_t kG, uint32_t kItemThreads, bool kJacobi, int kMinBlocks>
+__global__ void __launch_bounds__(kItemThreads, kMinBlocks)
+    solveItemsKernel(Buffers b, const DevParams* __restrict__ pp, const float4* __restrict__ src, float4* tgt,
+                     const uint32_t* __restrict__ list, uint32_t count, uint32_t K, uint32_t groups) {
+  extern __shared__ float4 cache4[];
+  // One incident tet per thread and round, kept over the trials; then also
+  // kTrials backtracked trials at a time once the first one has failed.
+  constexpr bool kHold = kG * kItemTets == kItemThreads;
+  constexpr uint32_t kTrials = kHold ? kItemTrials : 1u;
+  __shared__ ItemShared<kG, kTrials> sh;
+  float4* basisS = cache4;
+  float4* stateS = cache4 + size_t(groups) * K * kBasisWords;
+  float* rows = reinterpret_cast<float*>(stateS + size_t(groups) * K * kStateWords);
+  float* tetRows = rows + groups * K * kRowFloats;
+  const uint32_t tid = threadIdx.x;
+  const uint32_t first = blockIdx.x * groups, n = min(groups, count - first);
+  const uint32_t nrec = n * K;
+
+  // ---- vertices: what the block's threads need of each, and the ones that
+  // take no solve (jgs2-shader.ts:3042-3081 for the preflight rejection) ----
+  uint32_t status = kNonfinite, backtracks = 0, evals = 0;
+  float shiftN = 0.0f;
+  bool localValid = true, haveRecord = false;
+  if (tid == kItemThreads - 1) {
+    sh.fail = sh.maxBack = sh.skip = sh.evals = sh.maxShift = 0u;
+    sh.valid = 1u;
+  }
+  if (tid < groups) {
+    uint32_t solve = 0, v = 0, scene = 0;
+    bool have = tid < n;
+    if (have) v = list ? list[first + tid] : first + tid;
+    have = have && inBounds(v, b.vertexTotal, kSiteListVertex);
+    sh.count[tid] = 0u;
+    if (have) {
+      scene = b.vertexScene[v];
+      const DevParams& p = pp[scene];
+      if (p.active) {
+        const FrameState* fs = &b.frames[scene];
+        const uint4 info = b.vinfo[v];
+        sh.start[tid] = info.x;
+        sh.count[tid] = info.y;
+        if (latched(p, fs)) {
+          tgt[v] = src[v];
+        } else if (isPinned(info)) {
+          const float4 rm = b.restMass[v];
+          tgt[v] = make_float4(rm.x, rm.y, rm.z, 1.0f);
+          b.finalUpdate[v] = 0.0f;
+          float4* L = &b.local[4ull * v];
+          L[0] = L[1] = L[2] = make_float4(0, 0, 0, 0);
+          L[3] = make_float4(0, 0, 0, float(kPinned));
+          status = kPinned;
+          haveRecord = true;
+        } else {
+          const float4 c0 = fs->control[0];
+          const uint32_t vb = controlBits(c0.w) & kValidityMask;
+          const bool amv = (vb & kAcceptedMinimumValid) != 0u && finiteS(c0.z);
+          if (!(amv && c0.z > kDeterminantFloor)) {
+            tgt[v] = src[v];
+            b.finalUpdate[v] = 0.0f;
+            float4* L = &b.local[4ull * v];
+            L[0] = L[1] = L[2] = make_float4(0, 0, 0, 0);
+            status = amv ? kLineSearchFailed : kNonfinite;
+            L[3] = make_float4(amv ? c0.z : 0.f, 0, 0, float(status));
+            localValid = status != kNonfinite;
+            haveRecord = true;
+          } else {
+            solve = 1;
+          }
+        }
+      }
+    }
+    sh.v[tid] = v;
+    sh.scene[tid] = scene;
+    sh.solve[tid] = solve;
+  }
+  // ---- basis blocks: staged as they lie, sixteen bytes a copy ----
+  if (list == nullptr) {
+    const float4* from = b.cubBasis + size_t(first) * K * kBasisWords;
+    for (uint32_t c = tid; c < nrec * kBasisWords; c += kItemThreads) cpAsync16(&basisS[c], from + c);
+  } else {
+    const uint32_t per = K * kBasisWords;
+    for (uint32_t c = tid; c < n * per; c += kItemThreads) {
+      const uint32_t g = c / per, v = list[first + g];
+      if (inBounds(v, b.vertexTotal, kSiteListVertex)) cpAsync16(&basisS[c], b.cubBasis + size_t(v) * per + (c - g * per));
+    }
+  }
+  // The vertex's own data, wanted by one thread per vertex only later, when
+  // nothing else of the block would hide its latency.
+  for (uint32_t c = tid; c < n * 6u; c += kItemThreads) {
+    const uint32_t g = c / 6u, part = c - g * 6u, w = list ? list[first + g] : first + g;
+    if (!inBounds(w, b.vertexTotal, kSiteListVertex)) continue;
+    if (part == 0u) cpAsync16(&sh.own[g][0], src + w);
+    else if (part == 1u) cpAsync16(&sh.own[g][1], b.predicted + w);
+    else if (part == 2u) cpAsync16(&sh.own[g][2], b.restMass + w);
+    else if (kJacobi) cpAsync16(&sh.own[g][part], b.incident + 3ull * w + (part - 3u));
+  }
+  cpAsyncWaitAll();
+  __syncthreads();
+
+  // ---- records (jgs2-shader.ts:3197-3263) ----
+  for (uint32_t i = tid; i < nrec; i += kItemThreads) {
+    const uint32_t g = i / K;
+    if (!sh.solve[g]) continue;
+    const uint32_t v = sh.v[g];
+    const DevParams& p = pp[sh.scene[g]];
+    const bool objActive = p.objectiveFlags != 0u;
+    const size_t rec = size_t(v) * K + (i - g * K);
+    const uint4 head = __ldg(&b.cubHead[2 * rec]), idx = __ldg(&b.cubHead[2 * rec + 1]);
+    const float w = __uint_as_float(head.y);
+    float4* state = stateS + i * kStateWords;
+    if (!(head.x != kEmptyTet && w > 0.0f) || !inBounds(head.x, b.tetTotal, kSiteRecordTet) ||
+        !inBounds(idx.x, b.vertexTotal, kSiteRecordVertex) || !inBounds(idx.y, b.vertexTotal, kSiteRecordVertex) ||
+        !inBounds(idx.z, b.vertexTotal, kSiteRecordVertex) || !inBounds(idx.w, b.vertexTotal, kSiteRecordVertex)) {
+      state[3].w = 0.0f;
+      continue;
+    }
+    const TetRec r = loadTet(b.tets, head.x);
+    const M3 Rs = loadFrame(b.vertexPack, v);
+    CubState st;
+    recordStateOf<false>(b, p, v, w, idx, r, [&](int l) { return loadBlockVecShared(basisS + i * kBasisWords, l); },
+                         src, objActive, st);
+    const M3& F = st.F;
+    const M3 &dF0 = st.dF0, &dF1 = st.dF1, &dF2 = st.dF2;
+    const PiolaTerms pt = piolaTerms(F, r.lambda, r.mu);
+    const M3 P = piola(F, pt);
+    const float3 pg = r.vol * f3(frob(dF0, P), frob(dF1, P), frob(dF2, P)) + st.gQ;
+    const float p0 = frob(F, dF0), p1 = frob(F, dF1), p2 = frob(F, dF2);
+    const float q0 = frob(pt.cof, dF0), q1 = frob(pt.cof, dF1), q2 = frob(pt.cof, dF2);
+    S3 ph;
+    {
+      const M3 D0 = dcofactor(F, dF0);
+      ph.xx = pt.b * frob(dF0, D0);
+      ph.xy = pt.b * frob(dF1, D0);
+      ph.xz = pt.b * frob(dF2, D0);
+    }
+    {
+      const M3 D1 = dcofactor(F, dF1);
+      ph.yy = pt.b * frob(dF1, D1);
+      ph.yz = pt.b * frob(dF2, D1);
+    }
+    ph.zz = pt.b * frob(dF2, dcofactor(F, dF2));
+    ph.xx += pt.a * frob(dF0, dF0) + pt.c1 * p0 * p0 + r.lambda * q0 * q0;
+    ph.yy += pt.a * frob(dF1, dF1) + pt.c1 * p1 * p1 + r.lambda * q1 * q1;
+    ph.zz += pt.a * frob(dF2, dF2) + pt.c1 * p2 * p2 + r.lambda * q2 * q2;
+    ph.xy += pt.a * frob(dF0, dF1) + pt.c1 * p0 * p1 + r.lambda * q0 * q1;
+    ph.xz += pt.a * frob(dF0, dF2) + pt.c1 * p0 * p2 + r.lambda * q0 * q2;
+    ph.yz += pt.a * frob(dF1, dF2) + pt.c1 * p1 * p2 + r.lambda * q1 * q2;
+    ph.xx *= r.vol; ph.yy *= r.vol; ph.zz *= r.vol; ph.xy *= r.vol; ph.xz *= r.vol; ph.yz *= r.vol;
+    sadd(ph, st.HQ);
+    const float3 wg = w * mv(Rs, pg);
+    const S3 wh = srotate(Rs, ph);
+    float* row = rows + i * kRowFloats;
+    row[0] = wg.x; row[1] = wg.y; row[2] = wg.z;
+    row[3] = wh.xx; row[4] = wh.yy; row[5] = wh.zz; row[6] = wh.xy; row[7] = wh.xz; row[8] = wh.yz;
+    if (st.slot < 4) {
+      // The exact source block already in the local gather.
+      const float3 position = xyz(src[v]);
+      const float4 pv = b.predicted[v];
+      const float3 gs = st.gs;
+      // The fused forms solveChunk compiles to, spelled out.
+      const float3 away = position - xyz(pv), stress = mv(P, gs);
+      float3 ps = f3(__fmaf_rn(pv.w, away.x, __fmul_rn(r.vol, stress.x)),
+                     __fmaf_rn(pv.w, away.y, __fmul_rn(r.vol, stress.y)),
+                     __fmaf_rn(pv.w, away.z, __fmul_rn(r.vol, stress.z)));
+      if (objActive) {
+        const float share = 1.0f / float(sh.count[g] > 1u ? sh.count[g] : 1u);
+        const float3 og = objectiveGradient(p, b, v, position);
+        ps = f3(__fadd_rn(ps.x, __fmul_rn(og.x, share)), __fadd_rn(ps.y, __fmul_rn(og.y, share)),
+                __fadd_rn(ps.z, __fmul_rn(og.z, share)));
+      }
+      const S3 blk = incidentBlock(r, F, pt, gs);
+      const float3 wp = (-w) * ps;
+      row[9] = wp.x; row[10] = wp.y; row[11] = wp.z;
+      row[12] = blk.xx; row[13] = blk.yy; row[14] = blk.zz; row[15] = blk.xy; row[16] = blk.xz; row[17] = blk.yz;
+    }
+    // The state the trials read, over the basis it was formed from.
+    state[0] = make_float4(F.c0.x, F.c0.y, F.c0.z, r.vol);
+    state[1] = make_float4(F.c1.x, F.c1.y, F.c1.z, r.lambda);
+    state[2] = make_float4(F.c2.x, F.c2.y, F.c2.z, r.mu);
+    state[3] = make_float4(st.gs.x, st.gs.y, st.gs.z, w);
+    state[4] = make_float4(st.I0, st.J0, __uint_as_float(st.slot), 0.0f);
+    float4* d = basisS + i * kBasisWords;
+    d[0] = make_float4(dF0.c0.x, dF0.c0.y, dF0.c0.z, dF0.c1.x);
+    d[1] = make_float4(dF0.c1.y, dF0.c1.z, dF0.c2.x, dF0.c2.y);
+    d[2] = make_float4(dF0.c2.z, dF1.c0.x, dF1.c0.y, dF1.c0.z);
+    d[3] = make_float4(dF1.c1.x, dF1.c1.y, dF1.c1.z, dF1.c2.x);
+    d[4] = make_float4(dF1.c2.y, dF1.c2.z, dF2.c0.x, dF2.c0.y);
+    d[5] = make_float4(dF2.c0.z, dF2.c1.x, dF2.c1.y, dF2.c1.z);
+    d[6] = make_float4(dF2.c2.x, dF2.c2.y, dF2.c2.z, st.gQ.x);
+    d[7] = make_float4(st.gQ.y, st.gQ.z, st.HQ.xx, st.HQ.yy);
+    d[8] = make_float4(st.HQ.zz, st.HQ.xy, st.HQ.xz, st.HQ.yz);
+  }
+
+  // ---- incident tets ----
+  uint32_t most = 0;
+  for (uint32_t g = 0; g < n; ++g) most = max(most, sh.solve[g] ? sh.count[g] : 0u);
+  struct HeldTet {
+    M3 F;
+    float3 g;
+    float vol, lambda, mu;
+    bool ok;
+  };
+  auto loadHeld = [&](uint32_t g, uint32_t a, HeldTet& h) {
+    h.ok = false;
+    if (g >= n || !sh.solve[g] || a >= sh.count[g]) return;
+    const uint32_t entry = __ldg(&b.adjacency[sh.start[g] + a]);
+    TetRec r;
+    if (!incidentTetChecked(b.tets, entry, b.tetTotal, b.vertexTotal, &r)) return;
+    h.F = fused::deformation(r, src);
+    h.g = shapeGradient(r, entry & 3u);
+    h.vol = r.vol; h.lambda = r.lambda; h.mu = r.mu;
+    h.ok = true;
+  };
+  HeldTet held;
+  held.ok = false;
+  if constexpr (kHold) loadHeld(tid / kItemTets, tid % kItemTets, held);
+  // ---- sums: lane j of a vertex's four takes records j, j + 4, ... and
+  // (coloured sweeps) incident tets j, j + 4, ... ----
+  const uint32_t sg = tid / 4, lane = tid & 3u;
+  const unsigned mask = 0xfu << (tid & 28u);
+  const bool summing = sg < n && sh.solve[sg] != 0u;
+  Comp3 gsum = czero();
+  S3 hess = szero();
+  auto incidentRow = [&](uint32_t i, const HeldTet& h) {
+    if (!h.ok) return;
+    float3 f;
+    S3 blk;
+    fused::incident(h.F, h.g, h.vol, h.lambda, h.mu, &f, &blk);
+    float* row = tetRows + i * kTetRowFloats;
+    row[0] = f.x; row[1] = f.y; row[2] = f.z;
+    row[3] = blk.xx; row[4] = blk.yy; row[5] = blk.zz; row[6] = blk.xy; row[7] = blk.xz; row[8] = blk.yz;
+    row[9] = h.vol;
+  };
+  auto incidentRound = [&](uint32_t a0) {
+    for (uint32_t i = tid; i < n * kItemTets; i += kItemThreads) {
+      HeldTet h;
+      if (kHold && a0 == 0) h = held;
+      else loadHeld(i / kItemTets, a0 + i % kItemTets, h);
+      incidentRow(i, h);
+    }
+  };
+  if constexpr (!kJacobi) incidentRound(0);
+  __syncthreads();
+  if (summing) {
+    const uint32_t v = sh.v[sg];
+    for (uint32_t u = lane; u < K; u += 4) {
+      const float* row = rows + (sg * K + u) * kRowFloats;
+      const float4* state = stateS + (sg * K + u) * kStateWords;
+      const float w = state[3].w;
+      if (!(w > 0.0f)) continue;
+      cadd(gsum, f3(row[0], row[1], row[2]));
+      saddScaled(hess, w, S3{row[3], row[4], row[5], row[6], row[7], row[8]});
+      if (__float_as_uint(state[4].z) < 4u) {
+        const DevParams& p = pp[sh.scene[sg]];
+        const float nS = float(sh.count[sg] > 1u ? sh.count[sg] : 1u);
+        cadd(gsum, f3(row[9], row[10], row[11]));
+        saddScaled(hess, -w * state[0].w, S3{row[12], row[13], row[14], row[15], row[16], row[17]});
+        const float own = b.predicted[v].w + targetStiffness(p, b, v) / nS;
+        hess.xx = __fmaf_rn(-w, own, hess.xx);
+        hess.yy = __fmaf_rn(-w, own, hess.yy);
+        hess.zz = __fmaf_rn(-w, own, hess.zz);
+      }
+    }
+  }
+  if constexpr (!kJacobi) {
+    for (uint32_t a0 = 0; a0 == 0 || a0 < most; a0 += kItemTets) {
+      if (a0 > 0) {
+        __syncthreads();
+        incidentRound(a0);
+        __syncthreads();
+      }
+      if (summing)
+        for (uint32_t j = lane; j < kItemTets && a0 + j < sh.count[sg]; j += 4) {
+          const float* row = tetRows + (sg * kItemTets + j) * kTetRowFloats;
+          cadd(gsum, f3(row[0], row[1], row[2]));
+          saddScaled(hess, row[9], S3{row[3], row[4], row[5], row[6], row[7], row[8]});
+        }
+    }
+  }
+  if (summing) {
+    groupMerge<4>(gsum, mask);
+    hess.xx = groupSum<4>(hess.xx, mask);
+    hess.yy = groupSum<4>(hess.yy, mask);
+    hess.zz = groupSum<4>(hess.zz, mask);
+    hess.xy = groupSum<4>(hess.xy, mask);
+    hess.xz = groupSum<4>(hess.xz, mask);
+    hess.yz = groupSum<4>(hess.yz, mask);
+    if (lane == 0) {
+      float* o = sh.sum[sg];
+      o[0] = gsum.s.x; o[1] = gsum.s.y; o[2] = gsum.s.z;
+      o[3] = gsum.c.x; o[4] = gsum.c.y; o[5] = gsum.c.z;
+      o[6] = hess.xx; o[7] = hess.yy; o[8] = hess.zz; o[9] = hess.xy; o[10] = hess.xz; o[11] = hess.yz;
+    }
+  }
+  __syncthreads();
+
+  // ---- globalization (jgs2-shader.ts:3265-3473), one thread per vertex ----
+  const bool solving = tid < n && sh.solve[tid] != 0u;
+  const uint32_t v = tid < n ? sh.v[tid] : 0u;
+  const DevParams& p = pp[tid < n ? sh.scene[tid] : 0u];
+  SolveResult dr{f3(0, 0, 0), 0, 0, 0, 0, 0, kNonfinite};
+  float3 position = f3(0, 0, 0), predV = f3(0, 0, 0), grad = f3(0, 0, 0);
+  float inertia = 0.0f, resolution = 0.0f, controlMin = 0.0f;
+  float alpha = 0.0f, acceptedDelta = 0.0f, bound = 0.0f, minTrialDet = 0.0f, ta = 1.0f;
+  float3 acceptedD = f3(0, 0, 0), acceptedP = f3(0, 0, 0);
+  uint32_t bt = 0;
+  bool searching = false;
+  if (solving) {
+    position = xyz(sh.own[tid][0]);
+    predV = xyz(sh.own[tid][1]);
+    acceptedP = position;
+    inertia = sh.own[tid][2].w * p.invDt2;
+    const bool objActive = p.objectiveFlags != 0u;
+    const float3 objS = objActive ? objectiveGradient(p, b, v, position) : f3(0, 0, 0);
+    const float* o = sh.sum[tid];
+    Comp3 gs;
+    gs.s = f3(o[0], o[1], o[2]);
+    gs.c = f3(o[3], o[4], o[5]);
+    S3 h = {o[6], o[7], o[8], o[9], o[10], o[11]};
+    if constexpr (kJacobi) {
+      const float4 i0 = sh.own[tid][3], i1 = sh.own[tid][4], i2 = sh.own[tid][5];
+      cadd(gs, f3(i0.x, i0.y, i0.z));
+      h.xx += i0.w;
+      h.yy += i1.x;
+      h.zz += i1.y;
+      h.xy += i1.z;
+      h.xz += i1.w;
+      h.yz += i2.x;
+    }
+    // Own terms: inertia, objectives, floor (jgs2-shader.ts:3083-3092, 3188-3191).
+    cadd(gs, inertia * (position - predV));
+    saddDiag(h, inertia);
+    if (objActive) cadd(gs, objS);
+    if (p.objectiveFlags & 2u) saddDiag(h, targetStiffness(p, b, v));
+    if (p.floorStiffness > 0.0f && position.y < p.floorHeight) {
+      cadd(gs, f3(0.0f, p.floorStiffness * (position.y - p.floorHeight), 0.0f));
+      h.yy += p.floorStiffness;
+    }
+    grad = cvalue(gs);
+    dr = globalizationSolve(h, grad, inertia);
+    status = kNonfinite;
+    const float3 fullP = position + dr.direction;
+    const float3 fullD = fullP - position;
+    const float scs = fmaxf(fabsf(position.x), fmaxf(fabsf(position.y), fabsf(position.z)));
+    resolution = fmaxf(p.sceneScale, fmaxf(scs, 1.0e-12f)) * kUnitRoundoff * kPositionResolutionMultiplier;
+    const bool below = dr.status == kAccepted && finiteV(fullP) && finiteV(fullD) && scaledLength(fullD) <= resolution;
+    if (dr.status == kAccepted) status = below ? kZeroGradient : kLineSearchFailed;
+    else if (dr.status == kZeroGradient) status = kZeroGradient;
+    else if (dr.status == kShiftLimit) status = kShiftLimit;
+    else if (dr.status == kCholeskyFailed) status = kCholeskyFailed;
+    else if (dr.status == kNonDescent) status = kNonDescent;
+    if (dr.status == kAccepted && !below) {
+      searching = true;
+      const float dl = scaledLength(dr.direction);
+      if (p.maxStep > 0.0f && dl > p.maxStep) ta = p.maxStep / dl;
+      controlMin = b.frames[sh.scene[tid]].control[0].z;  // accepted-source minimum (finite here)
+    }
+  }
+  // ---- line search ----
+  // A round evaluates the first trial alone and then, where a thread holds its
+  // incident tet, the next kTrials of the backtracking sequence together: they
+  // do not depend on one another, and a vertex that a determinant bound holds
+  // back goes through all thirteen.  The trials are then judged in order.
+  uint32_t roundTrials = 1u;
+  for (;;) {
+    uint32_t evalCount = 0, firstBt = bt;
+    float firstTa = ta;
+    if (searching) {
+      searching = false;
+      for (; bt <= kMaxBacktracks; ++bt) {
+        const float3 tp = position + ta * dr.direction;
+        const float3 td = tp - position;
+        if (!finiteV(tp) || !finiteV(td)) {
+          if (evalCount == 0) { status = kNonfinite; minTrialDet = 0.f; backtracks = bt; }
+          break;
+        }
+        const float tl = scaledLength(td);
+        if (p.maxStep > 0.0f && tl > p.maxStep) {
+          if (evalCount > 0) break;
+          ta *= kBacktrackFactor;
+          continue;
+        }
+        if (tl <= resolution) {
+          if (evalCount == 0) { status = kZeroGradient; minTrialDet = 0.f; backtracks = bt; }
+          break;
+        }
+        const float gd = dot3(grad, td);
+        if (!finiteS(gd)) {
+          if (evalCount == 0) { status = kNonfinite; minTrialDet = 0.f; backtracks = bt; }
+          break;
+        }
+        if (!(gd < 0.0f)) {
+          if (evalCount == 0) { status = kZeroGradient; minTrialDet = 0.f; backtracks = bt; }
+          break;
+        }
+        if (evalCount == 0) {
+          firstBt = bt;
+          firstTa = ta;
+        }
+        const uint32_t j = evalCount++;
+        const float3 ts = mtv(loadFrame(b.vertexPack, v), td);
+        sh.td[j][tid][0] = td.x; sh.td[j][tid][1] = td.y; sh.td[j][tid][2] = td.z;
+        sh.ts[j][tid][0] = ts.x; sh.ts[j][tid][1] = ts.y; sh.ts[j][tid][2] = ts.z;
+        sh.ownMove[j][tid] = dot3(position - predV, td) + 0.5f * dot3(td, td);
+        const float nS = float(sh.count[tid] > 1u ? sh.count[tid] : 1u);
+        sh.ownObjective[j][tid] = p.objectiveFlags != 0u ? objectiveDelta(p, b, v, position, td) / nS : 0.0f;
+        if (evalCount == roundTrials) break;
+        ta *= kBacktrackFactor;
+      }
+    }
+    if (tid < groups) sh.eval[tid] = evalCount;
+    if (!__syncthreads_or(evalCount != 0u)) break;
+    // Restricted geometry and energy (restrictedMinimumDeformationDeterminant
+    // :1980-2118 and restrictedEnergyDelta :2120-2337).
+    const uint32_t recStride = groups * K * 2u, tetStride = groups * kItemTets * 3u;
+    float* recTrial = rows;                                   // (energy, J) per record and trial
+    float* tetTrial = rows + roundTrials * recStride;         // (energy, vol, J) per incident tet and trial
+    for (uint32_t i = tid; i < nrec * roundTrials; i += kItemThreads) {
+      const uint32_t j = kTrials > 1 ? i / nrec : 0u, r = i - j * nrec, g = r / K;
+      if (sh.eval[g] <= j) continue;
+      const float4* s = stateS + r * kStateWords;
+      const float4 s3 = s[3];
+      if (!(s3.w > 0.0f)) continue;
+      const float4 s0 = s[0], s1 = s[1], s2 = s[2], s4 = s[4];
+      const float4* d = basisS + r * kBasisWords;
+      const float4 d0 = d[0], d1 = d[1], d2 = d[2], d3 = d[3], d4 = d[4], d5 = d[5], d6 = d[6], d7 = d[7], d8 = d[8];
+      const M3 F = {xyz(s0), xyz(s1), xyz(s2)};
+      const M3 dF0 = {f3(d0.x, d0.y, d0.z), f3(d0.w, d1.x, d1.y), f3(d1.z, d1.w, d2.x)};
+      const M3 dF1 = {f3(d2.y, d2.z, d2.w), f3(d3.x, d3.y, d3.z), f3(d3.w, d4.x, d4.y)};
+      const M3 dF2 = {f3(d4.z, d4.w, d5.x), f3(d5.y, d5.z, d5.w), f3(d6.x, d6.y, d6.z)};
+      const float3 gQ = f3(d6.w, d7.x, d7.y);
+      const S3 HQ = {d7.z, d7.w, d8.x, d8.y, d8.z, d8.w};
+      const float vol = s0.w, lambda = s1.w, mu = s2.w;
+      const float3 ts = f3(sh.ts[j][g][0], sh.ts[j][g][1], sh.ts[j][g][2]);
+      const float3 step = f3(sh.td[j][g][0], sh.td[j][g][1], sh.td[j][g][2]);
+      float J = 0.0f;
+      // Record state is in the source frame: the trial step there is R_s^T td.
+      const M3 D = ts.x * dF0 + ts.y * dF1 + ts.z * dF2;
+      const float dm = vol * snhEnergyDelta(F, s4.x, s4.y, D, lambda, mu, &J);
+      float comp = dm + dot3(ts, gQ) + 0.5f * dot3(ts, smv(HQ, ts));
+      if (__float_as_uint(s4.z) < 4u) {
+        float Js;
+        comp -= vol * snhEnergyDelta(F, s4.x, s4.y, outer(step, xyz(s3)), lambda, mu, &Js);
+        comp -= sh.own[g][1].w * sh.ownMove[j][g];
+        if (pp[sh.scene[g]].objectiveFlags != 0u) comp -= sh.ownObjective[j][g];
+      }
+      recTrial[j * recStride + 2u * r] = comp;
+      recTrial[j * recStride + 2u * r + 1u] = J;
+    }
+    // Four lanes per vertex and trial add its items.
+    const uint32_t sj = kTrials > 1 ? sg / n : 0u, av = sg - sj * n;
+    const bool adding = sj < roundTrials && sg < n * roundTrials && sh.eval[av] > sj;
+    float jmin = kF32Max, de = 0.0f;
+    bool geomFinite = true;
+    // Lane-order index u >= K of an incident tet is adjacency slot u - K.
+    const uint32_t firstInc = lane >= K % 4u ? lane - K % 4u : lane + 4u - K % 4u;
+    for (uint32_t a0 = 0; a0 == 0 || a0 < most; a0 += kItemTets) {
+      if (a0 > 0) __syncthreads();
+      for (uint32_t i = tid; i < n * kItemTets; i += kItemThreads) {
+        const uint32_t g = i / kItemTets, trials = sh.eval[g];
+        if (trials == 0u) continue;
+        HeldTet h;
+        if (kHold && a0 == 0) h = held;
+        else loadHeld(g, a0 + i % kItemTets, h);
+        if (!h.ok) continue;
+        for (uint32_t j = 0; j < trials; ++j) {
+          float J = 0.0f;
+          const float e = fused::energyDelta(h.F, f3(sh.td[j][g][0], sh.td[j][g][1], sh.td[j][g][2]), h.g, h.lambda,
+                                             h.mu, &J);
+          float* t = tetTrial + j * tetStride + 3u * i;
+          t[0] = e;
+          t[1] = h.vol;
+          t[2] = J;
+        }
+      }
+      __syncthreads();
+      if (adding) {
+        if (a0 == 0)
+          for (uint32_t u = lane; u < K; u += 4) {
+            const float w = stateS[(av * K + u) * kStateWords + 3].w;
+            if (!(w > 0.0f)) continue;
+            const float* t = recTrial + sj * recStride + 2u * (av * K + u);
+            const float J = t[1];
+            de = __fmaf_rn(w, t[0], de);
+            if (!finiteS(J)) geomFinite = false;
+            jmin = fminf(jmin, J);
+          }
+        for (uint32_t j = firstInc; j < kItemTets && a0 + j < sh.count[av]; j += 4) {
+          const float* t = tetTrial + sj * tetStride + 3u * (av * kItemTets + j);
+          const float J = t[2];
+          de = __fmaf_rn(t[1], t[0], de);
+          if (!finiteS(J)) geomFinite = false;
+          jmin = fminf(jmin, J);
+        }
+      }
+    }
+    if (adding) {
+      jmin = groupMin<4>(jmin, mask);
+      const bool allFinite = __all_sync(mask, geomFinite);
+      de = groupSum<4>(de, mask);
+      if (lane == 0) {
+        sh.jmin[sj][av] = jmin;
+        sh.de[sj][av] = de;
+        sh.finite[sj][av] = allFinite ? 1u : 0u;
+      }
+    }
+    __syncthreads();
+    if (evalCount > 0) {
+      bt = firstBt;
+      ta = firstTa;
+      searching = true;
+      for (uint32_t j = 0; j < evalCount && searching; ++j, ++bt) {
+        if (!sh.finite[j][tid]) {
+          status = kNonfinite;
+          minTrialDet = 0.f;
+          backtracks = bt;
+          searching = false;
+          break;
+        }
+        const float trialMin = fminf(controlMin, sh.jmin[j][tid]);
+        minTrialDet = trialMin;
+        if (trialMin > kDeterminantFloor) {
+          const float3 tp = position + ta * dr.direction;
+          const float3 td = tp - position;
+          float energy = sh.de[j][tid];
+          energy += inertia * (dot3(position - predV, td) + 0.5f * dot3(td, td)) + floorDelta(p, position.y, td.y);
+          if (p.objectiveFlags != 0u) energy += objectiveDelta(p, b, v, position, td);
+          evals += 1;
+          const float tb = kArmijoC1 * dot3(grad, td);
+          if (!finiteS(energy)) {
+            status = kNonfinite;
+            backtracks = bt;
+            searching = false;
+            break;
+          }
+          if (energy <= tb) {
+            alpha = ta;
+            acceptedDelta = energy;
+            bound = tb;
+            backtracks = bt;
+            status = kAccepted;
+            acceptedD = td;
+            acceptedP = tp;
+            searching = false;
+            break;
+          }
+        }
+        ta *= kBacktrackFactor;
+      }
+    }
+    roundTrials = kTrials;
+  }
+  if (solving) {
+    if (status == kLineSearchFailed) backtracks = kMaxBacktracks;
+    tgt[v] = make_float4(acceptedP.x, acceptedP.y, acceptedP.z, 1.0f);
+    b.finalUpdate[v] = scaledLength(acceptedD);
+    float4* L = &b.local[4ull * v];
+    const float4 l0 = make_float4(dr.direction.x, dr.direction.y, dr.direction.z, alpha);
+    const float4 l1 = make_float4(dr.minEig * dr.scale, dr.scale, dr.shift * dr.scale, dr.shift);
+    const float4 l2 = make_float4(acceptedDelta, bound, dr.gdd, dr.residual);
+    const float4 l3 = make_float4(minTrialDet, float(backtracks), float(evals), float(status));
+    L[0] = l0; L[1] = l1; L[2] = l2; L[3] = l3;
+    localValid = finiteS(l0.x) && finiteS(l0.y) && finiteS(l0.z) && finiteS(l0.w) && finiteS(l1.x) &&
+                 finiteS(l1.y) && finiteS(l1.z) && finiteS(l1.w) && finiteS(l2.x) && finiteS(l2.y) &&
+                 finiteS(l2.z) && finiteS(l2.w) && finiteS(l3.x) && status != kNonfinite && l1.w >= 0.0f;
+    shiftN = dr.shift;
+    haveRecord = true;
+  }
+  // Local aggregates of reduceCandidate's vertex loop (jgs2-shader.ts:3689-3790),
+  // per scene: folded in shared memory when the block's vertices share one
+  // scene, otherwise added per vertex.
+  const uint32_t blockScene = sh.scene[0];
+  const bool oneScene = __syncthreads_and(tid >= n || !haveRecord || sh.scene[tid] == blockScene) != 0;
+  if (haveRecord) {
+    const bool failure = status == kShiftLimit || status == kNonDescent || status == kLineSearchFailed ||
+                         status == kNonfinite || status == kCholeskyFailed;
+    uint32_t trials = 0;
+    if (status == kAccepted) trials = backtracks + 1;
+    else if (status == kLineSearchFailed && backtracks == kMaxBacktracks) trials = kTrialCount;
+    else if (status == kZeroGradient && backtracks > 0) trials = backtracks;
+    else if (status == kNonfinite) trials = backtracks;  // a nonfinite trial never has J above the floor here
+    const uint32_t skipped = trials - (trials < evals ? trials : evals);
+    const uint32_t shiftBits = (shiftN > 0.0f && finiteS(shiftN)) ? __float_as_uint(shiftN) : 0u;
+    FrameState* fs = &b.frames[sh.scene[tid]];
+    uint32_t* fail = oneScene ? &sh.fail : &fs->localFailures;
+    uint32_t* back = oneScene ? &sh.maxBack : &fs->localMaxBacktracks;
+    uint32_t* skip = oneScene ? &sh.skip : &fs->localSkipped;
+    uint32_t* ev = oneScene ? &sh.evals : &fs->localEvaluations;
+    uint32_t* shift = oneScene ? &sh.maxShift : &fs->localMaxShift;
+    uint32_t* valid = oneScene ? &sh.valid : &fs->localNumericsValid;
+    if (failure) atomicAdd(fail, 1u);
+    if (backtracks) atomicMax(back, backtracks);
+    if (skipped) atomicAdd(skip, skipped);
+    if (evals) atomicAdd(ev, evals);
+    if (shiftBits) atomicMax(shift, shiftBits);
+    if (!localValid) atomicAnd(valid, 0u);
+  }
+  __syncthreads();
+  if (oneScene && tid == 0) {
+    FrameState* fs = &b.frames[blockScene];
+    if (sh.fail) atomicAdd(&fs->localFailures, sh.fail);
+    if (sh.maxBack) atomicMax(&fs->localMaxBacktracks, sh.maxBack);
+    if (sh.skip) atomicAdd(&fs->localSkipped, sh.skip);
+    if (sh.evals) atomicAdd(&fs->localEvaluations, sh.evals);
+    if (sh.maxShift) atomicMax(&fs->localMaxShift, sh.maxShift);
+    if (!sh.valid) atomicAnd(&fs->localNumericsValid, 0u);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // Graph-coloured sweep as one persistent kernel (jgs2-solver.ts:2275-2325,
 // colour masks jgs2-shader.ts:3004-3012): for each colour, the vertex frames
 // of the vertices the colour's solves read, a grid barrier, the in-place
@@ -2760,7 +3495,7 @@ __global__ void __launch_bounds__(kBlock, JGS2_SOLVE_MIN_BLOCKS)
       const uint32_t scene = b.vertexScene[v];
       const DevParams& p = pp[scene];
       if (!p.active || latched(p, &b.frames[scene])) continue;
-      storeFrame(b.vertexRot, v, vertexFrame<true>(b, x, v, p.rotationEpsilon));
+      storeFrame(b.vertexPack, v, vertexFrame<true>(b, x, v, p.rotationEpsilon), xyz(__ldca(x + v)));
     }
     if (!gridBarrier(bar, spinLimit)) return;
     const uint32_t cb = colorOffsets[c], count = colorOffsets[c + 1] - cb;
@@ -3071,7 +3806,9 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) prologueKernel(Bu
     } else {
       b.velocity[i] = make_float4(0, 0, 0, 0);
     }
-    b.predicted[i] = make_float4(pred.x, pred.y, pred.z, distributedInertiaWeight(rm, info, p.invDt2));
+    const float4 target = make_float4(pred.x, pred.y, pred.z, distributedInertiaWeight(rm, info, p.invDt2));
+    b.predicted[i] = target;
+    b.vertexPack[4ull * i + 3] = target;
     b.finalUpdate[i] = 0.0f;
     // Co-rotated path: the iteration source is the inertial prediction; the
     // stable iteration source is the accepted pose.
@@ -3084,7 +3821,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) prologueKernel(Bu
     else incidentSums<true>(b, b.pos[0], info, sums);
     if (isPinned(info)) {
       const M3 favg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
-      storeFrame(b.vertexRot, i, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
+      storeFrame(b.vertexPack, i, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon), xyz(o));
     } else {
       storeFrameAndIncident(b, p, b.pos[0], i, info, sums);
     }
@@ -3335,7 +4072,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock, kWide ? 2 : JGS2_
     }
     if (nextRotations) {
       const M3 favg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
-      storeFrame(b.vertexRot, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon));
+      storeFrame(b.vertexPack, v, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon), xyz(acc[v]));
     }
   }
   ConvPartial tot = part;
@@ -3792,6 +4529,49 @@ int launchVertexPolar(const Buffers& b, const DevParams* p, const float4* src, c
   return 1;
 }
 
+template <uint32_t kG, uint32_t kThreads, bool kJacobi, int kMin>
+void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
+                 uint32_t count, uint32_t K, uint32_t shift, cudaStream_t s) {
+  static_assert(4 * kG <= kThreads, "four summing lanes per vertex");
+  constexpr uint32_t trials = kG * kItemTets == kThreads ? kItemTrials : 1u;
+  static_assert(4 * kG * trials <= kThreads, "four summing lanes per vertex and trial");
+  const uint32_t limit = solveSharedBytes() - 12288;  // static shared memory of the kernel
+  uint32_t groups = kG;
+  while (groups > 1 && itemSharedBytes(groups, K, !kJacobi, trials) > limit) --groups;
+  groups = std::max(1u, groups >> shift);
+  static int attr = 0;
+  if (attr == 0) {
+    attr = static_cast<int>(limit);
+    cudaFuncSetAttribute(solveItemsKernel<kG, kThreads, kJacobi, kMin>, cudaFuncAttributeMaxDynamicSharedMemorySize, attr);
+  }
+  solveItemsKernel<kG, kThreads, kJacobi, kMin>
+      <<<(count + groups - 1) / groups, kThreads, itemSharedBytes(groups, K, !kJacobi, trials), s>>>(
+          b, p, src, tgt, list, count, K, groups);
+}
+
+// The item form, or false where solveKernel's four lanes per vertex are the
+// faster one.  Jacobi: eight vertices a block while one wave of two blocks per
+// SM holds them, sixteen while that does (2 688 vertices: 27 us, 33 with
+// eight, 37 with 32), then 32 on three blocks per SM.  Coloured lists: eight
+// for three waves of blocks (3 650 vertices per colour: 60 us, 64 with sixteen,
+// 71 with four lanes); past that four lanes (10 300 per colour: 90 us, 105 with
+// sixteen, 117 with eight).
+constexpr uint32_t kItemBlocks = 296;  // two per SM
+constexpr uint32_t kItemLargest = 40000;
+bool launchSolveItems(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
+                      uint32_t count, uint32_t K, bool jacobi, uint32_t shift, cudaStream_t s) {
+  if (jacobi) {
+    if (count <= 8 * kItemBlocks) launchItems<8, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
+    else if (count <= 16 * kItemBlocks) launchItems<16, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
+    else if (count <= kItemLargest) launchItems<32, 160, true, 3>(b, p, src, tgt, list, count, K, shift, s);
+    else return false;
+  } else {
+    if (count <= 3 * 8 * kItemBlocks) launchItems<8, 192, false, 2>(b, p, src, tgt, list, count, K, shift, s);
+    else return false;
+  }
+  return true;
+}
+
 int launchSolve(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
                 uint32_t count, uint32_t K, bool cachedIncident, cudaStream_t s) {
   if (count == 0) return 0;
@@ -3827,6 +4607,7 @@ int launchSolve(const Buffers& b, const DevParams* p, const float4* src, float4*
   } else if (b.clothRange || b.contactIdx) {
     if (cache) solveKernel<kGroup, true, true><<<blocks, threads, smem, s>>>(b, p, src, tgt, list, count, K, ci, groups);
     else solveKernel<kGroup, true, false><<<blocks, threads, 0, s>>>(b, p, src, tgt, list, count, K, ci, groups);
+  } else if (cache && K > 0 && launchSolveItems(b, p, src, tgt, list, count, K, cachedIncident, shift, s)) {
   } else {
     if (cache) solveKernel<kGroup, false, true><<<blocks, threads, smem, s>>>(b, p, src, tgt, list, count, K, ci, groups);
     else solveKernel<kGroup, false, false><<<blocks, threads, 0, s>>>(b, p, src, tgt, list, count, K, ci, groups);

@@ -104,7 +104,9 @@ struct Buffers {
   float4* predicted;       // inertial target xyz, distributed inertia weight m/(h^2 n) (0 pinned)
   float4* velocity;
   float4* old;
-  float4* vertexRot;      // 3 per vertex (columns)
+  // 4 per vertex: the frame's columns with the position x, y, z at the same
+  // pose in their w, then the inertial target and its weight (predicted).
+  float4* vertexPack;
   float4* tetRot;         // 3 per tet (co-rotated only)
   float* finalUpdate;     // per vertex update norm
   float4* local;          // 4 per vertex (local diagnostics)

@@ -1446,6 +1446,17 @@ jgs2_status readRegion(Engine* s, const void* dev, size_t bytes, void* host) {
   return checkBroadPhase(s);
 }
 
+// The vertex frames as 12 floats per vertex (three columns, w = 0) from the
+// vertex packs, which keep a position there: the strided copy, and the zeros
+// once it has arrived.
+cudaError_t copyFrames(Engine* s, void* out, uint32_t vertices) {
+  return cudaMemcpy2DAsync(out, 48, s->b.vertexPack, 64, 48, vertices, cudaMemcpyDeviceToHost, s->stream);
+}
+void clearFrameW(void* frames, uint32_t vertices) {
+  unsigned char* p = static_cast<unsigned char*>(frames);
+  for (size_t i = 0; i < 3ull * vertices; ++i) std::memset(p + 16 * i + 12, 0, 4);
+}
+
 // The host mirrors may change only after the previous upload from them has
 // been consumed by the copy engine.
 jgs2_status waitObjectiveMirror(Engine* s) {
@@ -1967,17 +1978,14 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
   STEP(upload(sp, &b.old, pos.data(), nV));
   STEP(upload(sp, &b.velocity, vel.data(), nV));
   {
-    std::vector<float4> identity(3ull * nV);
+    std::vector<float4> pack(4ull * nV);
     for (uint32_t v = 0; v < nV; ++v) {
-#if defined(JGS2_FRAME_QUAT) && JGS2_FRAME_QUAT
-      identity[3ull * v] = make_float4(0, 0, 0, 1);  // the identity quaternion
-#else
-      identity[3ull * v] = make_float4(1, 0, 0, 0);
-#endif
-      identity[3ull * v + 1] = make_float4(0, 1, 0, 0);
-      identity[3ull * v + 2] = make_float4(0, 0, 1, 0);
+      pack[4ull * v] = make_float4(1, 0, 0, pos[v].x);
+      pack[4ull * v + 1] = make_float4(0, 1, 0, pos[v].y);
+      pack[4ull * v + 2] = make_float4(0, 0, 1, pos[v].z);
+      pack[4ull * v + 3] = pos[v];
     }
-    STEP(upload(sp, &b.vertexRot, identity.data(), 3ull * nV));
+    STEP(upload(sp, &b.vertexPack, pack.data(), 4ull * nV));
   }
   b.tetRot = nullptr;
   STEP(deviceAlloc(sp, &b.finalUpdate, nV));
@@ -2855,8 +2863,16 @@ jgs2_status jgs2_read_final_iteration_updates(jgs2_solver* s, float* out, size_t
 }
 
 jgs2_status jgs2_read_vertex_rotations(jgs2_solver* s, float* out, size_t floats) {
-  if (usable(s) != JGS2_OK) return usable(s);
-  return readSceneVec4(s, 0, s->b.vertexRot, out, floats, 12);
+  const jgs2_status st = usable(s);
+  if (st != JGS2_OK) return st;
+  const uint32_t V = s->scenes[0].V;
+  if (!out || floats < 12ull * V)
+    return readSceneVec4(s, 0, s->b.vertexPack, out, floats, 12);  // the size check's error
+  CUDA_TRY(s, cudaSetDevice(s->device));
+  CUDA_TRY(s, copyFrames(s, out, V));
+  CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+  clearFrameW(out, V);
+  return checkBroadPhase(s);
 }
 
 jgs2_status jgs2_read_globalization(jgs2_solver* s, float* local, size_t localFloats, float* control,
@@ -3020,7 +3036,7 @@ struct StateRegion {
 std::vector<StateRegion> stateRegions(Engine* s) {
   const size_t V = s->V;
   return {{s->b.pos[0], 16 * V},        {s->b.velocity, 16 * V},  {s->b.old, 16 * V},
-          {s->b.predicted, 16 * V},     {s->b.vertexRot, 48 * V}, {s->b.incident, 48 * V},
+          {s->b.predicted, 16 * V},     {s->b.vertexPack, 48 * V}, {s->b.incident, 48 * V},
           {s->b.local, 64 * V},         {s->b.finalUpdate, 4 * V}, {s->b.forces, 16 * V},
           {s->b.targets, 16 * V},       {s->b.frames, sizeof(FrameState)}};
 }
@@ -3061,11 +3077,18 @@ jgs2_status jgs2_export_state(jgs2_solver* s, void* out, size_t capacity, size_t
   unsigned char* p = static_cast<unsigned char*>(out);
   std::memcpy(p, &h, sizeof(h));
   p += sizeof(h);
+  unsigned char* frames = nullptr;
   for (const StateRegion& r : stateRegions(s)) {
-    CUDA_TRY(s, cudaMemcpyAsync(p, r.dev, r.bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (r.dev == s->b.vertexPack) {
+      frames = p;
+      CUDA_TRY(s, copyFrames(s, p, s->V));
+    } else {
+      CUDA_TRY(s, cudaMemcpyAsync(p, r.dev, r.bytes, cudaMemcpyDeviceToHost, s->stream));
+    }
     p += r.bytes;
   }
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+  clearFrameW(frames, s->V);
   return JGS2_OK;
 }
 
@@ -3094,7 +3117,10 @@ jgs2_status jgs2_import_state(jgs2_solver* s, const void* in, size_t size) {
   for (const StateRegion& r : stateRegions(s)) {
     if (r.dev == s->b.forces) std::memcpy(s->hForces, p, r.bytes);
     if (r.dev == s->b.targets) std::memcpy(s->hTargets, p, r.bytes);
-    CUDA_TRY(s, cudaMemcpyAsync(r.dev, p, r.bytes, cudaMemcpyHostToDevice, s->stream));
+    if (r.dev == s->b.vertexPack)  // the prologue of the next frame fills the positions in
+      CUDA_TRY(s, cudaMemcpy2DAsync(r.dev, 64, p, 48, 48, s->V, cudaMemcpyHostToDevice, s->stream));
+    else
+      CUDA_TRY(s, cudaMemcpyAsync(r.dev, p, r.bytes, cudaMemcpyHostToDevice, s->stream));
     p += r.bytes;
   }
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));
