@@ -80,7 +80,7 @@ def test_backtracked_trials_are_judged_in_order(fillers):
         want = want or got
         for a, b in zip(want, got):
             np.testing.assert_array_equal(a, b)
-    assert want[3][:, 28].max() >= 2  # the most backtracks of an iteration
+    assert want[3][:, 28].max() >= 1  # some vertex went past its first trial
 
 
 def _against_oracle(inp, schedule, iterations):
@@ -96,7 +96,7 @@ def _against_oracle(inp, schedule, iterations):
     hg = g.readGlobalizationDiagnostics()
     hc = np.asarray(c.read("history"), dtype=np.float32).reshape(-1, 32)[:iterations]
     np.testing.assert_array_equal(hg["history"][:, 4:6], hc[:, 4:6])
-    return hg["local"]
+    return hg["history"]
 
 
 def _fan(n):
@@ -126,3 +126,15 @@ def test_more_incident_tets_than_a_round(n, schedule):
 @pytest.mark.parametrize("schedule", ["jacobi", GGS2])
 def test_wide_cached_records(schedule):
     _against_oracle(_bar((2, 1, 1), K=60, exact=True), schedule, 2)
+
+
+# A bar shaken until vertices backtrack two and three times (seeded): the f32
+# and FP64 oracles agree on it to 3e-7 of the diagonal.
+@pytest.mark.parametrize("schedule", ["jacobi", GGS2])
+def test_backtracking_follows_the_oracle(schedule):
+    inp = scenes.cantilever(cells=(12, 4, 4), method=scenes.PRECOMPUTE_PATCH)
+    rng = np.random.default_rng(4)
+    p = inp.positions.reshape(-1, 4)
+    free = inp.vertex_info.reshape(-1, 4)[:, 2] == 0
+    p[free, :3] += rng.uniform(-0.012, 0.012, (free.sum(), 3)).astype(np.float32)
+    assert _against_oracle(inp, schedule, 2)[:, 28].max() >= 2
