@@ -21,7 +21,7 @@ constexpr uint32_t kIpcVertexTriangle = 0u, kIpcEdgeEdge = 1u;
 
 enum ContactSlot : int {
   kContactSource = 0, kContactSourceWeights = 1, kContactTarget = 2, kContactTargetWeights = 3,
-  kContactLagged = 4, kContactLaggedWeights = 5, kContactScratch = 6, kContactStateWords = 7,
+  kContactLagged = 4, kContactLaggedWeights = 5, kContactStateWords = 6,
 };
 
 struct ContactData {
@@ -393,6 +393,16 @@ __device__ __forceinline__ ContactData ipcCached(float4 nd, float4 w) {
   return {valid ? nd.w : 0.0f, valid ? f3(nd.x, nd.y, nd.z) : f3(1, 0, 0), valid ? w : make_float4(0, 0, 0, 0),
           valid};
 }
+
+// What most passes need of a cached contact, in four bytes instead of the
+// state's 96: its distance, with the sign bit set when the candidate carries
+// lagged friction, or NaN when the cache is invalid.  A pass reads the state
+// only of the candidates that this word does not settle.
+__device__ __forceinline__ float ipcNear(bool valid, float distance, bool friction) {
+  return valid ? copysignf(distance, friction ? -1.0f : 1.0f) : __int_as_float(0x7fffffff);
+}
+__device__ __forceinline__ bool ipcNearValid(float near) { return near == near; }
+__device__ __forceinline__ bool ipcNearFriction(float near) { return signbit(near); }
 
 // ipcStoreCachedContact (jgs2-shader.ts:378-406).
 __device__ __forceinline__ void ipcStoreCached(float4* state, int slot, const ContactData& k) {

@@ -1086,7 +1086,7 @@ __device__ __forceinline__ bool contactPinnedMotion(const Buffers& b, uint4 q, c
 // cross, frictionless and free of unbounded pinned motion.  The decision
 // depends on the candidate only, so every incident vertex agrees.
 __device__ __forceinline__ bool contactIncluded(const Buffers& b, const DevParams& p, uint32_t c,
-                                                const float4* __restrict__ src) {
+                                                const float4* __restrict__ src, float* near) {
   const float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
   const ContactData k = ipcCached(st[kContactSource], st[kContactSourceWeights]);
   const bool friction = p.ipcFriction > 0.0f && st[kContactLagged].w > 0.0f;
@@ -1095,6 +1095,7 @@ __device__ __forceinline__ bool contactIncluded(const Buffers& b, const DevParam
   uint32_t type;
   const uint4 q = contactIndices(b, c, &type);
   const bool pinnedMotion = contactPinnedMotion(b, q, src, fmaxf(p.maxStep, 0.0f));
+  *near = ipcNear(k.valid, k.distance, friction);
   return !k.valid || !bounded || k.distance <= reach || friction || pinnedMotion;
 }
 
@@ -1127,18 +1128,56 @@ __device__ __forceinline__ float contactEnergy(const Buffers& b, const DevParams
   return e;
 }
 
+// A lane's walk over a vertex's active candidates (`ids` at a, a + stride, ...):
+// the ids and their near words are fetched four ahead, so that the walk does
+// not wait for two dependent loads per candidate.
+struct ContactBatch {
+  uint32_t c0, c1, c2, c3;
+  float d0, d1, d2, d3;
+  uint32_t left = 0;
+  __device__ __forceinline__ float next(const uint32_t* __restrict__ ids, const float* __restrict__ near, uint32_t a,
+                                        uint32_t n, uint32_t stride, uint32_t* c) {
+    if (left == 0) {
+      c0 = ids[a];
+      c1 = ids[min(a + stride, n - 1)];
+      c2 = ids[min(a + 2 * stride, n - 1)];
+      c3 = ids[min(a + 3 * stride, n - 1)];
+      d0 = near[c0];
+      d1 = near[c1];
+      d2 = near[c2];
+      d3 = near[c3];
+      left = 4;
+    }
+    *c = c0;
+    const float d = d0;
+    c0 = c1; c1 = c2; c2 = c3;
+    d0 = d1; d1 = d2; d2 = d3;
+    --left;
+    return d;
+  }
+};
+
 // ipcLocalContribution (:788-869) over the vertex's active candidates
 // [first, count) step `stride`: barrier gradient and PSD normal block, lagged
 // friction gradient and tangential block.  `fresh` evaluates the contact at x
-// (the coloured schedule), otherwise the cache at `slot` is used.
+// (the coloured schedule), otherwise the cache at `slot` is used, whose
+// distances are in `near`.
 template <bool kHessian, class G>
 __device__ __forceinline__ void contactLocal(const Buffers& b, const DevParams& p, uint32_t v,
-                                             const float4* __restrict__ x, bool fresh, int slot, uint32_t first,
-                                             uint32_t stride, G& grad, S3& hess) {
+                                             const float4* __restrict__ x, bool fresh, int slot,
+                                             const float* __restrict__ near, uint32_t first, uint32_t stride, G& grad,
+                                             S3& hess) {
   const uint2 range = b.contactRange[v];
   const uint32_t n = b.activeCount[v];
+  ContactBatch batch;
   for (uint32_t a = first; a < n; a += stride) {
-    const uint32_t c = b.activeIds[range.x + a];
+    uint32_t c;
+    if (fresh) {
+      c = b.activeIds[range.x + a];
+    } else {
+      const float d = batch.next(b.activeIds + range.x, near, a, n, stride, &c);
+      if (!ipcNearValid(d) || !(ipcBarrierActive(fabsf(d), p.ipcActivation) || ipcNearFriction(d))) continue;
+    }
     const float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
     const ContactData k = fresh ? contactAt(b, c, x, p.ipcActivation) : ipcCached(st[slot], st[slot + 1]);
     if (!k.valid) continue;
@@ -1212,7 +1251,6 @@ __global__ void JGS2_CONTACT_BOUNDS contactLagKernel(Buffers b, const DevParams*
   }
   st[kContactLagged] = force;
   st[kContactLaggedWeights] = w;
-  st[kContactScratch] = make_float4(1, 0, 0, 0);
   if (c == b.scenes[scene].kOff) b.frames[scene].contactAlpha = 1.0f;
 }
 
@@ -1233,7 +1271,9 @@ __global__ void __launch_bounds__(kBlock) contactFlagKernel(Buffers b, const Dev
     fs->checkAlphaBits = __float_as_uint(1.0f);
     fs->checkValid = 1u;
   }
-  b.contactFlag[c] = contactIncluded(b, p, c, src) ? 1u : 0u;
+  float near;
+  b.contactFlag[c] = contactIncluded(b, p, c, src, &near) ? 1u : 0u;
+  b.contactNear[c] = near;
 }
 
 // ...then, one warp per vertex, the ordered compaction of its included
@@ -1247,13 +1287,26 @@ __global__ void __launch_bounds__(kBlock) contactRowsKernel(Buffers b, const Dev
   if (!p.active || !p.ipc) return;
   const uint2 r = b.contactRange[v];
   uint32_t n = 0;
-  for (uint32_t k0 = 0; k0 < r.y; k0 += 32) {
-    const uint32_t k = k0 + lane;
-    const uint32_t c = k < r.y ? b.contactIds[r.x + k] : 0u;
-    const bool keep = k < r.y && b.contactFlag[c] != 0u;
-    const unsigned ballot = __ballot_sync(0xffffffffu, keep);
-    if (keep) b.activeIds[r.x + n + __popc(ballot & ((1u << lane) - 1u))] = c;
-    n += __popc(ballot);
+  // Eight rounds of 32 candidates in flight: a vertex of the reference's trough
+  // has about 1 400, and one round at a time (an index, then its flag) took
+  // 39 us.
+  constexpr uint32_t kAhead = 8;
+  for (uint32_t k0 = 0; k0 < r.y; k0 += 32 * kAhead) {
+    uint32_t c[kAhead];
+    bool keep[kAhead];
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) {
+      const uint32_t k = k0 + 32 * j + lane;
+      c[j] = k < r.y ? b.contactIds[r.x + k] : 0u;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) keep[j] = k0 + 32 * j + lane < r.y && b.contactFlag[c[j]] != 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) {
+      const unsigned ballot = __ballot_sync(0xffffffffu, keep[j]);
+      if (keep[j]) b.activeIds[r.x + n + __popc(ballot & ((1u << lane) - 1u))] = c[j];
+      n += __popc(ballot);
+    }
   }
   if (lane == 0) b.activeCount[v] = n;
 }
@@ -1277,7 +1330,8 @@ __global__ void __launch_bounds__(kBlock) contactGradientKernel(Buffers b, const
   const int slot = (accepted && finiteS(alpha) && alpha > 0.0f) ? kContactTarget : kContactSource;
   float3 g = f3(0, 0, 0);
   S3 unused = szero();
-  contactLocal<false>(b, p, v, accepted ? tgt : src, false, slot, lane, 32u, g, unused);
+  contactLocal<false>(b, p, v, accepted ? tgt : src, false, slot,
+                      slot == kContactTarget ? b.contactTargetNear : b.contactNear, lane, 32u, g, unused);
   g.x = groupSum<32>(g.x, 0xffffffffu);
   g.y = groupSum<32>(g.y, 0xffffffffu);
   g.z = groupSum<32>(g.z, 0xffffffffu);
@@ -1286,7 +1340,19 @@ __global__ void __launch_bounds__(kBlock) contactGradientKernel(Buffers b, const
 
 __device__ __forceinline__ uint32_t alphaBits(float a) { return a > 0.0f ? __float_as_uint(a) : 0u; }
 
-// candidateContactStep of one candidate.
+// Each vertex's step length this iteration, or -1 when the step is not finite
+// (the candidate is then invalid whatever the other lengths are).
+__global__ void __launch_bounds__(kBlock) contactMoveKernel(Buffers b, const float4* __restrict__ src,
+                                                            const float4* __restrict__ tgt, uint32_t V) {
+  const uint32_t v = blockIdx.x * kBlock + threadIdx.x;
+  if (v >= V) return;
+  const float3 d = xyz(tgt[v]) - xyz(src[v]);
+  b.contactMove[v] = finiteV(d) ? length3(d) : -1.0f;
+}
+
+// candidateContactStep of one candidate.  kMoves: the step lengths come from
+// contactMoveKernel, four 4-byte gathers instead of eight of 16 bytes.
+template <bool kMoves>
 __device__ __forceinline__ void contactStepOne(const Buffers& b, const DevParams* __restrict__ pp,
                                                const float4* __restrict__ src, const float4* __restrict__ tgt,
                                                uint32_t c) {
@@ -1294,30 +1360,35 @@ __device__ __forceinline__ void contactStepOne(const Buffers& b, const DevParams
   const DevParams& p = pp[scene];
   if (!p.active || !p.ipc) return;
   FrameState* fs = &b.frames[scene];
-  float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
-  if (latched(p, fs)) {
-    st[kContactScratch] = make_float4(1, 0, 0, 1);
-    return;  // alpha one, valid: the reduction's identity
-  }
+  if (latched(p, fs)) return;  // alpha one, valid: the reduction's identity
   uint32_t type;
   const uint4 q = contactIndices(b, c, &type);
-  const float3 d0 = xyz(tgt[q.x]) - xyz(src[q.x]), d1 = xyz(tgt[q.y]) - xyz(src[q.y]);
-  const float3 d2 = xyz(tgt[q.z]) - xyz(src[q.z]), d3 = xyz(tgt[q.w]) - xyz(src[q.w]);
-  float L = 0.0f;
-  if (type == kIpcVertexTriangle) L = length3(d0) + fmaxf(length3(d1), fmaxf(length3(d2), length3(d3)));
-  else L = fmaxf(length3(d0), length3(d1)) + fmaxf(length3(d2), length3(d3));
-  ContactData source = ipcCached(st[kContactSource], st[kContactSourceWeights]);
-  bool fullStepSafe = source.valid && finiteS(L) && source.distance - L > p.ipcMinDistance;
-  if (!fullStepSafe) {
-    source = contactAt(b, c, src, kF32Max);
-    fullStepSafe = source.valid && finiteS(L) && source.distance - L > p.ipcMinDistance;
+  float l0, l1, l2, l3;
+  bool trialValid;
+  if (kMoves) {
+    const float m0 = b.contactMove[q.x], m1 = b.contactMove[q.y], m2 = b.contactMove[q.z], m3 = b.contactMove[q.w];
+    l0 = m0; l1 = m1; l2 = m2; l3 = m3;
+    trialValid = m0 >= 0.0f && m1 >= 0.0f && m2 >= 0.0f && m3 >= 0.0f;
+  } else {
+    const float3 d0 = xyz(tgt[q.x]) - xyz(src[q.x]), d1 = xyz(tgt[q.y]) - xyz(src[q.y]);
+    const float3 d2 = xyz(tgt[q.z]) - xyz(src[q.z]), d3 = xyz(tgt[q.w]) - xyz(src[q.w]);
+    l0 = length3(d0); l1 = length3(d1); l2 = length3(d2); l3 = length3(d3);
+    trialValid = finiteV(d0) && finiteV(d1) && finiteV(d2) && finiteV(d3);
   }
-  const bool trialValid = finiteV(d0) && finiteV(d1) && finiteV(d2) && finiteV(d3);
-  const bool valid = source.valid && trialValid && source.distance > p.ipcMinDistance && finiteS(L);
+  const float L = type == kIpcVertexTriangle ? l0 + fmaxf(l1, fmaxf(l2, l3)) : fmaxf(l0, l1) + fmaxf(l2, l3);
+  const float near = b.contactNear[c];
+  bool sourceValid = ipcNearValid(near);
+  float distance = fabsf(near);
+  bool fullStepSafe = sourceValid && finiteS(L) && distance - L > p.ipcMinDistance;
+  if (!fullStepSafe) {
+    const ContactData source = contactAt(b, c, src, kF32Max);
+    sourceValid = source.valid;
+    distance = source.distance;
+    fullStepSafe = sourceValid && finiteS(L) && distance - L > p.ipcMinDistance;
+  }
+  const bool valid = sourceValid && trialValid && distance > p.ipcMinDistance && finiteS(L);
   float alpha = 0.0f;
-  if (valid) alpha = fullStepSafe ? 1.0f : ipcSafeStepCap(source.distance, p.ipcMinDistance, L, p.ipcSafety);
-  st[kContactScratch] = make_float4(alpha, source.valid ? source.distance : 0.0f,
-                                    trialValid ? source.distance : 0.0f, valid ? 1.0f : 0.0f);
+  if (valid) alpha = fullStepSafe ? 1.0f : ipcSafeStepCap(distance, p.ipcMinDistance, L, p.ipcSafety);
   if (valid && finiteS(alpha)) {
     if (alpha < 1.0f) atomicMin(&fs->stepAlphaBits, alphaBits(alpha));
   } else {
@@ -1328,12 +1399,13 @@ __device__ __forceinline__ void contactStepOne(const Buffers& b, const DevParams
 
 // candidateContactStep (:2784-2847) with the min / all-valid reduction of
 // reduceContactStep folded in as order-free atomics.
+template <bool kMoves>
 __global__ void JGS2_CONTACT_BOUNDS contactStepKernel(Buffers b, const DevParams* __restrict__ pp,
                                                             const float4* __restrict__ src,
                                                             const float4* __restrict__ tgt) {
   const uint32_t n = contactListed(b);
   for (uint32_t c = blockIdx.x * kBlock + threadIdx.x; c < n; c += gridDim.x * kBlock)
-    contactStepOne(b, pp, src, tgt, c);
+    contactStepOne<kMoves>(b, pp, src, tgt, c);
 }
 
 // applyContactStep (:2909-2917): candidate = source + alpha (candidate -
@@ -1371,9 +1443,9 @@ __global__ void JGS2_CONTACT_BOUNDS contactValidateKernel(Buffers b, const DevPa
     const ContactData k = contactAt(b, c, tgt, p.ipcActivation + contactRoundingReach(p));
     float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
     ipcStoreCached(st, kContactTarget, k);
+    const ContactData stored = ipcCached(st[kContactTarget], st[kContactTargetWeights]);
+    b.contactTargetNear[c] = ipcNear(stored.valid, stored.distance, ipcNearFriction(b.contactNear[c]));
     const bool valid = k.valid && finiteS(k.distance) && k.distance > p.ipcMinDistance;
-    const float d = valid ? k.distance : 0.0f;
-    st[kContactScratch] = make_float4(1.0f, d, d, valid ? 1.0f : 0.0f);
     if (!valid) {
       atomicMin(&fs->checkAlphaBits, 0u);
       atomicAnd(&fs->checkValid, 0u);
@@ -1417,6 +1489,7 @@ __global__ void __launch_bounds__(kBlock) contactPromoteKernel(Buffers b, const 
       float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
       st[kContactSource] = st[kContactTarget];
       st[kContactSourceWeights] = st[kContactTargetWeights];
+      b.contactNear[c] = b.contactTargetNear[c];
     }
   }
 }
@@ -1441,6 +1514,7 @@ __global__ void __launch_bounds__(kBlock) contactPromoteKernel(Buffers b, const 
 // row keeps ascending candidate order, as the static rows do.
 
 constexpr uint32_t kBpChunk = 32;
+constexpr uint32_t kBpKept = kBpRowHits;
 constexpr uint32_t kBpClosedMax = 64;  // closed one-ring vertices a row keeps in shared memory
 constexpr float kBpInf = __builtin_huge_valf();
 
@@ -1621,9 +1695,14 @@ __global__ void JGS2_CONTACT_BOUNDS bpInitKernel(Buffers b, const DevParams* __r
     const uint32_t prev = first ? 0xffffffffu : b.bpPrev[c];
     float4 s0, s1;
     if (prev != 0xffffffffu) {
+      // promoteAcceptedContactCache (:2694-2710) of the previous iteration: the
+      // target contacts of an accepted pose become the source cache.
+      const FrameState* fs = &b.frames[b.contactScene[c]];
+      const float alpha = fs->contactAlpha;
+      const int slot = fs->control[1].x == 1.0f && finiteS(alpha) && alpha > 0.0f ? kContactTarget : kContactSource;
       const float4* ps = b.bpPrevState + kContactStateWords * static_cast<size_t>(prev);
-      s0 = ps[kContactSource];
-      s1 = ps[kContactSourceWeights];
+      s0 = ps[slot];
+      s1 = ps[slot + 1];
       lagF = ps[kContactLagged];
       lagW = ps[kContactLaggedWeights];
       st[kContactSource] = s0;
@@ -1644,10 +1723,10 @@ __global__ void JGS2_CONTACT_BOUNDS bpInitKernel(Buffers b, const DevParams* __r
     }
     st[kContactLagged] = lagF;
     st[kContactLaggedWeights] = lagW;
-    st[kContactScratch] = make_float4(1, 0, 0, 0);
     // contactIncluded on the state just written.
     const ContactData k = ipcCached(s0, s1);
     const bool friction = p.ipcFriction > 0.0f && lagF.w > 0.0f;
+    b.contactNear[c] = ipcNear(k.valid, k.distance, friction);
     const bool bounded = p.maxStep > 0.0f;
     const float reach = p.ipcActivation + 2.0f * (fmaxf(p.maxStep, 0.0f) + contactRoundingReach(p));
     const bool pinnedMove =
@@ -1657,13 +1736,14 @@ __global__ void JGS2_CONTACT_BOUNDS bpInitKernel(Buffers b, const DevParams* __r
     const uint32_t key = b.bpSentinel;
     reinterpret_cast<uint4*>(b.bpKeys[0])[c] =
         active ? make_uint4(q.x, q.y, q.z, q.w) : make_uint4(key, key, key, key);
-    reinterpret_cast<uint4*>(b.bpVals[0])[c] = make_uint4(c, c, c, c);
   }
 }
 
 // One warp per row: the row's pairs in column order, counted (kWrite false,
 // into bpRowOff[row]) or placed at the row's offset with their previous
-// entry (kWrite true).  The columns are walked 32 superchunks (of 32 chunks
+// entry (kWrite true).  The count keeps a row's first kBpKept hit chunks with
+// their masks, from which the write pass places the pairs without testing any
+// box; a row with more walks them again.  The columns are walked 32 superchunks (of 32 chunks
 // of 32 primitives) at a time, then 32 chunks, then 32 primitives, each
 // level only inside the boxes the row's box does not clear.
 template <bool kWrite>
@@ -1681,16 +1761,82 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
   const DevParams& p = pp[scene];
   uint32_t count = 0;
   if (p.active && p.ipc && row.z < row.w) {
-    const float reach = bpReach(p);
     uint32_t rv[2];
-    BpBox P;
     if (edgeRow) {
       const uint2 e = b.bpEdges[row.x];
       rv[0] = e.x;
       rv[1] = e.y;
-      P = bpLoad(b.bpEdgeBox, row.x);
     } else {
       rv[0] = rv[1] = row.x;
+    }
+    const uint32_t base = kWrite ? b.bpRowOff[r] : 0u;
+    uint32_t pc = 0, pe = 0;  // this row's entries of the previous list
+    if (!first) {
+      pc = b.bpPrevRowOff[r];
+      pe = b.bpPrevRowOff[r + 1];
+    }
+    // Carry cursor: the previous entries [qc, qc + 64), in w0 and w1.
+    uint32_t qc = pc;
+    uint32_t w0 = 0xffffffffu, w1 = 0xffffffffu;
+    if (kWrite && !first) {
+      if (pc + lane < pe) w0 = b.bpPrevCols[pc + lane];
+      if (pc + 32 + lane < pe) w1 = b.bpPrevCols[pc + 32 + lane];
+    }
+    // Places the hits `m` of a chunk (this lane's column `col`, hit or not).
+    auto place = [&](uint32_t chunk, unsigned m) {
+      const uint32_t col = chunk * kBpChunk + lane;
+      const bool hit = (m >> lane) & 1u;
+      // The previous list's entries of this chunk (sorted, at most 32):
+      // a bit per column, so a listed pair finds its entry by rank.  The
+      // entries are read 64 at a time and kept over the chunks.
+      uint32_t prev = 0xffffffffu;
+      if (!first) {
+        const uint32_t chunkStart = chunk * kBpChunk;
+        while (qc < pe && __shfl_sync(0xffffffffu, w0, 31) < chunkStart) {
+          qc += 32;
+          w0 = w1;
+          w1 = qc + 32 + lane < pe ? b.bpPrevCols[qc + 32 + lane] : 0xffffffffu;
+        }
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, w0 < chunkStart));
+        const uint32_t o0 = w0 - chunkStart, o1 = w1 - chunkStart;
+        const unsigned have = __reduce_or_sync(0xffffffffu, (o0 < kBpChunk ? (1u << o0) : 0u) |
+                                                                (o1 < kBpChunk ? (1u << o1) : 0u));
+        if ((have >> lane) & 1u) prev = qc + below + __popc(have & ((1u << lane) - 1u));
+      }
+      if (hit) {
+        const uint32_t pos = base + count + __popc(m & ((1u << lane) - 1u));
+        uint4 q;
+        if (edgeRow) {
+          const uint2 e = b.bpEdges[col];
+          q = make_uint4(rv[0], rv[1], e.x, e.y | 0x80000000u);
+        } else {
+          const uint4 t = b.bpTris[col];
+          q = make_uint4(rv[0], t.x, t.y, t.z);
+        }
+        b.contactIdx[pos] = q;
+        b.contactScene[pos] = scene;
+        b.bpCols[pos] = col;
+        b.bpPrev[pos] = prev;
+      }
+      count += __popc(m);
+    };
+    // The count pass keeps a row's hit chunks with their masks, up to 32, so
+    // that the write pass need not test the boxes again.
+    uint32_t kept = 0;
+    uint2 mine = make_uint2(0u, 0u);
+    if constexpr (kWrite) {
+      const uint32_t n = b.bpRowKept[r];
+      if (n <= kBpKept) {
+        if (lane < n) mine = b.bpRowHits[static_cast<size_t>(r) * kBpKept + lane];
+        for (uint32_t i = 0; i < n; ++i) place(__shfl_sync(0xffffffffu, mine.x, i), __shfl_sync(0xffffffffu, mine.y, i));
+        return;
+      }
+    }
+    const float reach = bpReach(p);
+    BpBox P;
+    if (edgeRow) {
+      P = bpLoad(b.bpEdgeBox, row.x);
+    } else {
       const uint32_t vs[1] = {row.x};
       P = bpPrimitive(b, p, src, vs);
     }
@@ -1732,13 +1878,6 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
       }
       return false;
     };
-    const uint32_t base = kWrite ? b.bpRowOff[r] : 0u;
-    uint32_t pc = 0, pe = 0;  // this row's entries of the previous list
-    if (!first) {
-      pc = b.bpPrevRowOff[r];
-      pe = b.bpPrevRowOff[r + 1];
-    }
-    uint32_t qc = pc;  // carry cursor: first previous entry at or past the current chunk
     const uint32_t chunkLo = row.z / kBpChunk, chunkHi = (row.w - 1) / kBpChunk;
     const float4* superBoxes = edgeRow ? b.bpEdgeSuper : b.bpTriSuper;
     const float4* chunkBoxes = edgeRow ? b.bpEdgeChunk : b.bpTriChunk;
@@ -1792,44 +1931,20 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
             if (!hit && !bpSeparated(P, bpLoad(primBoxes, col), reach)) hit = !closed(col);
           }
           const unsigned m = __ballot_sync(0xffffffffu, hit);
-          if (kWrite && m) {
-            // The previous list's entries of this chunk (sorted, at most 32):
-            // a bit per column, so a listed pair finds its entry by rank.
-            uint32_t prev = 0xffffffffu;
-            if (!first) {
-              const uint32_t chunkStart = (c0 + j) * kBpChunk;
-              while (qc < pe) {
-                const uint32_t i = qc + lane;
-                const unsigned below = __ballot_sync(0xffffffffu, i < pe && b.bpPrevCols[i] < chunkStart);
-                qc += __popc(below);
-                if (below != 0xffffffffu) break;
-              }
-              const uint32_t i = qc + lane;
-              const uint32_t pcol = i < pe ? b.bpPrevCols[i] : 0xffffffffu;
-              const uint32_t off = pcol - chunkStart;
-              const unsigned have = __reduce_or_sync(0xffffffffu, off < kBpChunk ? (1u << off) : 0u);
-              if ((have >> lane) & 1u) prev = qc + __popc(have & ((1u << lane) - 1u));
-            }
-            if (hit) {
-              const uint32_t pos = base + count + __popc(m & ((1u << lane) - 1u));
-              uint4 q;
-              if (edgeRow) {
-                const uint2 e = b.bpEdges[col];
-                q = make_uint4(rv[0], rv[1], e.x, e.y | 0x80000000u);
-              } else {
-                const uint4 t = b.bpTris[col];
-                q = make_uint4(rv[0], t.x, t.y, t.z);
-              }
-              b.contactIdx[pos] = q;
-              b.contactScene[pos] = scene;
-              b.bpCols[pos] = col;
-              b.bpPrev[pos] = prev;
-            }
+          if constexpr (kWrite) {
+            if (m) place(c0 + j, m);
+          } else if (m) {
+            if (lane == kept) mine = make_uint2(c0 + j, m);
+            ++kept;
+            count += __popc(m);
           }
-          count += __popc(m);
         }
         __syncwarp();  // carried[] is rewritten by the next window
       }
+    }
+    if constexpr (!kWrite) {
+      if (lane < kept) b.bpRowHits[static_cast<size_t>(r) * kBpKept + lane] = mine;
+      if (lane == 0) b.bpRowKept[r] = kept;
     }
   }
   if (!kWrite && lane == 0) b.bpRowOff[r] = count;
@@ -1837,30 +1952,49 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
 
 constexpr int kScanThreads = 1024;
 
-// Exclusive scan of data[0, n) in place by one block of kScanThreads threads
-// (a contiguous run per thread); returns the total.  With the total above
-// `limit` every entry becomes zero.
+// Exclusive scan of data[0, n) in place by one block of kScanThreads threads;
+// returns the total.  With the total above `limit` every entry becomes zero.
+// Each warp takes a contiguous run 32 entries at a time, eight rounds in
+// flight (a run per thread, entry after entry, took 60 us for 65 000 rows).
 __device__ uint64_t blockScan(uint32_t* data, uint32_t n, uint64_t limit) {
-  __shared__ uint64_t part[kScanThreads];
-  const uint32_t per = (n + kScanThreads - 1) / kScanThreads;
-  const uint32_t lo = min(n, threadIdx.x * per), hi = min(n, lo + per);
+  constexpr uint32_t kWarps = kScanThreads / 32, kAhead = 8;
+  __shared__ uint64_t part[kWarps];
+  const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31u;
+  const uint32_t per = ((n + kWarps - 1) / kWarps + 31u) & ~31u;
+  const uint32_t lo = min(n, warp * per), hi = min(n, lo + per);
   uint64_t s = 0;
-  for (uint32_t i = lo; i < hi; ++i) s += data[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (uint32_t o = 1; o < kScanThreads; o <<= 1) {
-    const uint64_t add = threadIdx.x >= o ? part[threadIdx.x - o] : 0ull;
-    __syncthreads();
-    part[threadIdx.x] += add;
-    __syncthreads();
+  for (uint32_t i0 = lo; i0 < hi; i0 += 32 * kAhead) {
+    uint32_t v[kAhead];
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) v[j] = i0 + 32 * j + lane < hi ? data[i0 + 32 * j + lane] : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) s += v[j];
   }
-  const uint64_t total = part[kScanThreads - 1];
+#pragma unroll
+  for (uint32_t o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) part[warp] = s;
+  __syncthreads();
+  uint64_t run = 0, total = 0;
+  for (uint32_t w = 0; w < kWarps; ++w) {
+    if (w == warp) run = total;
+    total += part[w];
+  }
   const bool over = total > limit;
-  uint64_t run = part[threadIdx.x] - s;
-  for (uint32_t i = lo; i < hi; ++i) {
-    const uint32_t c = data[i];
-    data[i] = over ? 0u : static_cast<uint32_t>(run);
-    run += c;
+  for (uint32_t i0 = lo; i0 < hi; i0 += 32 * kAhead) {
+    uint32_t v[kAhead];
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) v[j] = i0 + 32 * j + lane < hi ? data[i0 + 32 * j + lane] : 0u;
+#pragma unroll
+    for (uint32_t j = 0; j < kAhead; ++j) {
+      uint32_t x = v[j];  // a run's sum may pass 32 bits only above the limit
+#pragma unroll
+      for (uint32_t o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (i0 + 32 * j + lane < hi) data[i0 + 32 * j + lane] = over ? 0u : static_cast<uint32_t>(run) + x - v[j];
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
   }
   __syncthreads();
   return total;
@@ -1939,6 +2073,9 @@ __global__ void __launch_bounds__(kScanThreads) bpSortScanKernel(const uint32_t*
   if (threadIdx.x == 0) hist[256u * tiles + blockIdx.x] = static_cast<uint32_t>(total);
 }
 
+// kFirst: the entries still lie four to a candidate, in candidate order, so
+// their values are not stored.
+template <bool kFirst>
 __global__ void __launch_bounds__(kSortThreads) bpSortScatterKernel(const uint32_t* __restrict__ kin,
                                                                     const uint32_t* __restrict__ vin,
                                                                     uint32_t* __restrict__ kout,
@@ -1999,25 +2136,30 @@ __global__ void __launch_bounds__(kSortThreads) bpSortScatterKernel(const uint32
       const uint32_t i = base + j * 32 + lane;
       const uint32_t o = digitBase[dig[j]] + hist[dig[j] * tiles + tile] + wh[w][dig[j]] + pos[j];
       kout[o] = kin[i];
-      vout[o] = vin[i];
+      vout[o] = kFirst ? i / 4u : vin[i];
     }
   }
 }
 
-// Each vertex's run of the sorted keys is its active row.
+// Each vertex's run of the sorted keys is its active row: the run's first
+// entry sets its start, and first and last add up its length (integers, on the
+// zero the boxes pass left).
 __global__ void __launch_bounds__(kBlock) bpSegmentsKernel(Buffers b, const uint32_t* __restrict__ keys) {
-  const uint32_t M = 4u * __ldcg(b.bpStatus);
-  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < M; i += gridDim.x * kBlock) {
-    const uint32_t k = keys[i];
-    if (k >= b.bpSentinel || (i > 0 && keys[i - 1] == k)) continue;
-    uint32_t lo = i + 1, hi = M;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (keys[mid] <= k) lo = mid + 1;
-      else hi = mid;
+  const uint32_t n = __ldcg(b.bpStatus);  // groups of four entries
+  for (uint32_t g = blockIdx.x * kBlock + threadIdx.x; g < n; g += gridDim.x * kBlock) {
+    const uint4 q = reinterpret_cast<const uint4*>(keys)[g];
+    const uint32_t before = g > 0 ? keys[4 * g - 1] : ~0u, after = g + 1 < n ? keys[4 * g + 4] : ~0u;
+    const uint32_t k[6] = {before, q.x, q.y, q.z, q.w, after};
+#pragma unroll
+    for (uint32_t j = 1; j <= 4; ++j) {
+      if (k[j] >= b.bpSentinel) continue;
+      const uint32_t i = 4 * g + j - 1;
+      if (k[j - 1] != k[j]) {
+        b.contactRange[k[j]] = make_uint2(i, 0u);
+        atomicSub(&b.activeCount[k[j]], i);
+      }
+      if (k[j + 1] != k[j]) atomicAdd(&b.activeCount[k[j]], i + 1);
     }
-    b.contactRange[k] = make_uint2(i, 0u);
-    b.activeCount[k] = lo - i;
   }
 }
 
@@ -2400,7 +2542,7 @@ __device__ __forceinline__ void solveChunk(const Buffers& b, const DevParams* __
         // ---- IPC contact (jgs2-shader.ts:3193-3195): the cached source
         // contacts, or fresh ones under the coloured schedule ----
         if (kExt && p.ipc)
-          contactLocal<true>(b, p, v, src, !cachedIncident, kContactSource, lane, W, gsum, hess);
+          contactLocal<true>(b, p, v, src, !cachedIncident, kContactSource, b.contactNear, lane, W, gsum, hess);
         // Group reduction of the gather.
         groupMerge<W>(gsum, mask);
         hess.xx = groupSum<W>(hess.xx, mask);
@@ -2574,8 +2716,20 @@ __device__ __forceinline__ void solveChunk(const Buffers& b, const DevParams* __
             // friction energy deltas (:2137-2196).
             if (kExt && contactActive) {
               const float dl = length3(td);
+              ContactBatch batch;
               for (uint32_t a = lane; a < contactActive; a += W) {
-                const uint32_t c = b.activeIds[contactFirst + a];
+                uint32_t c;
+                if (!cachedIncident) {
+                  c = b.activeIds[contactFirst + a];
+                } else {
+                  const float near = batch.next(b.activeIds + contactFirst, b.contactNear, a, contactActive, W, &c);
+                  if (!ipcNearValid(near)) {
+                    geomFinite = false;
+                    continue;
+                  }
+                  const float left = fabsf(near) - dl;
+                  if (left > p.ipcMinDistance && !(left < p.ipcActivation) && !ipcNearFriction(near)) continue;
+                }
                 const float4* cst = b.contactState + kContactStateWords * static_cast<size_t>(c);
                 const ContactData source = cachedIncident ? ipcCached(cst[kContactSource], cst[kContactSourceWeights])
                                                           : contactAt(b, c, src, p.ipcActivation);
@@ -3733,6 +3887,10 @@ __device__ __forceinline__ void accumulateContact(GatePartial& acc, const Buffer
                                                   float contactAlpha, uint32_t c, const float4* __restrict__ src,
                                                   const float4* __restrict__ tgt) {
   if (!b.contactFlag[c]) return;  // not in the active rows of this iteration
+  const float near = b.contactNear[c], after = contactAlpha != 0.0f ? b.contactTargetNear[c] : near;
+  if (ipcNearValid(near) && ipcNearValid(after) && !ipcNearFriction(near) &&
+      !ipcBarrierActive(fabsf(near), p.ipcActivation) && !ipcBarrierActive(fabsf(after), p.ipcActivation))
+    return;  // neither pose touches it: both energies are zero
   const float4* st = b.contactState + kContactStateWords * static_cast<size_t>(c);
   const ContactData ks = ipcCached(st[kContactSource], st[kContactSourceWeights]);
   const ContactData kc = contactAlpha != 0.0f ? ipcCached(st[kContactTarget], st[kContactTargetWeights]) : ks;
@@ -4746,7 +4904,13 @@ uint32_t candidateBlocks(const Buffers& b) {
 
 int launchContactStep(const Buffers& b, const DevParams* p, const float4* src, const float4* tgt, cudaStream_t s) {
   if (b.contactCount == 0) return 0;
-  contactStepKernel<<<candidateBlocks(b), kBlock, 0, s>>>(b, p, src, tgt);
+  // Lists of many candidates a vertex: the lengths once per vertex first.
+  if (b.contactDynamic) {
+    contactMoveKernel<<<blocksFor(b.vertexTotal), kBlock, 0, s>>>(b, src, tgt, b.vertexTotal);
+    contactStepKernel<true><<<candidateBlocks(b), kBlock, 0, s>>>(b, p, src, tgt);
+    return 2;
+  }
+  contactStepKernel<false><<<candidateBlocks(b), kBlock, 0, s>>>(b, p, src, tgt);
   return 1;
 }
 
@@ -4802,10 +4966,11 @@ int launchBroadPhase(const Buffers& b, const DevParams* p, const float4* src, ui
     const uint32_t in = pass & 1u, out = in ^ 1u;
     bpSortHistKernel<<<tiles, kSortThreads, 0, s>>>(b.bpKeys[in], b.bpStatus, 8u * pass, b.bpHist);
     bpSortScanKernel<<<256, kScanThreads, 0, s>>>(b.bpStatus, b.bpHist);
-    bpSortScatterKernel<<<tiles, kSortThreads, 0, s>>>(b.bpKeys[in], b.bpVals[in], b.bpKeys[out], b.bpVals[out],
-                                                       b.bpStatus, 8u * pass, b.bpHist);
+    const auto scatter = pass == 0 ? bpSortScatterKernel<true> : bpSortScatterKernel<false>;
+    scatter<<<tiles, kSortThreads, 0, s>>>(b.bpKeys[in], b.bpVals[in], b.bpKeys[out], b.bpVals[out], b.bpStatus,
+                                           8u * pass, b.bpHist);
   }
-  const uint32_t segBlocks = std::min(blocksFor(4u * b.contactCount), smCount() * 8u);
+  const uint32_t segBlocks = std::min(blocksFor(b.contactCount), smCount() * 16u);
   bpSegmentsKernel<<<segBlocks, kBlock, 0, s>>>(b, b.bpKeys[b.bpSortPasses & 1u]);
   return 7 + 3 * static_cast<int>(b.bpSortPasses);
 }

@@ -69,11 +69,17 @@ struct RedBlock {
 // 14.6).  From 1.2 M elements on longer blocks fold fewer partials.
 //   Prologue and convergence: entries of kConvChunk vertices, one warp each.
 constexpr uint32_t kGateMinChunk = 128, kGateMaxChunk = 2048, kGateBlocksPerScene = 592;
-inline uint32_t gateChunk(uint32_t elements) {
+// Contact surfaces: at most 512, since a listed candidate costs a thread more
+// than a tet (2.7 M listed: gate 218 us at 2 048, 123 at 1 024, 126 at 512;
+// a quarter of them: 117, 68, 44).
+constexpr uint32_t kGateListedChunk = 512;
+inline uint32_t gateChunk(uint32_t elements, bool listed) {
   const uint32_t per = (elements / kGateBlocksPerScene + kGateMinChunk - 1) / kGateMinChunk * kGateMinChunk;
-  return per < kGateMinChunk ? kGateMinChunk : per > kGateMaxChunk ? kGateMaxChunk : per;
+  const uint32_t most = listed ? kGateListedChunk : kGateMaxChunk;
+  return per < kGateMinChunk ? kGateMinChunk : per > most ? most : per;
 }
 constexpr uint32_t kConvChunk = 32;
+constexpr uint32_t kBpRowHits = 32;  // hit chunks a broad-phase row keeps from its count to its write
 
 // Reduction scratch and the GPU-resident control/history records
 // (dynamic arena regions globalizationControl/globalizationHistory,
@@ -147,7 +153,7 @@ struct Buffers {
   const uint32_t* clothIncidence;
   // IPC contact (all null without candidates): per candidate its global
   // vertex indices with the type (1 = edge-edge) in bit 31 of the fourth, its
-  // scene and 7 float4 of state (jgs2_contact.cuh); per vertex the range
+  // scene and 6 float4 of state (jgs2_contact.cuh); per vertex the range
   // (first, count) of its incident candidates in `contactIds` and the count
   // of active ones, listed at the same offsets in `activeIds`.
   uint4* contactIdx;
@@ -158,6 +164,9 @@ struct Buffers {
   uint32_t* activeCount;
   uint32_t* activeIds;
   uint32_t* contactFlag;   // per candidate: active this iteration
+  float* contactNear;        // per candidate: ipcNear of its source cache this iteration
+  float* contactTargetNear;  // ... and of its target cache
+  float* contactMove;        // per vertex: its step length (broad phase)
   float4* contactGrad;     // per vertex: IPC gradient at the accepted pose
   uint32_t gateBlocks, convBlocks, sceneCount, contactCount;
   uint32_t vertexTotal, tetTotal;  // vertices and tets over the scenes (checked builds bound indices by them)
@@ -194,6 +203,8 @@ struct Buffers {
   float4* bpEdgeSuper;
   uint32_t* bpRowOff;
   const uint32_t* bpPrevRowOff;
+  uint2* bpRowHits;     // kBpRowHits per row: (chunk, hit mask) of the iteration's count
+  uint32_t* bpRowKept;  // hit chunks of the row
   uint32_t* bpCols;
   const uint32_t* bpPrevCols;
   const float4* bpPrevState;

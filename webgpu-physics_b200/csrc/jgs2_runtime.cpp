@@ -1220,7 +1220,9 @@ int encodeFrame(Engine* s, uint32_t iterations, uint32_t schedule, bool bodyCorr
       n += timed(P::kContact, [&] { return jgs2::launchContactGradient(b, s->dParams, src, tgt, s->V, st); });
     n += timed(P::kConvergence,
                [&] { return jgs2::launchConvergence(b, s->dParams, src, tgt, !colored && !last, st); });
-    if (contact) n += timed(P::kContact, [&] { return jgs2::launchContactPromote(b, s->dParams, st); });
+    // Within the frame the broad phase promotes as it carries the cache over.
+    if (contact && (!dynamic || last))
+      n += timed(P::kContact, [&] { return jgs2::launchContactPromote(b, s->dParams, st); });
   }
   const float4* finalPos = (iterations % 2 == 0) ? s->b.pos[1] : s->b.pos[0];
   n += timed(P::kEpilogue,
@@ -1957,7 +1959,7 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
     const uint32_t n = std::max(std::max(std::max(sc.V, sc.T), std::max(sc.C, sc.H)), std::max(sc.KC, listed));
     r.gateSpan = std::max(n, 1u);
     r.gateBase = static_cast<uint32_t>(gateTable.size());
-    const uint32_t gateChunk = jgs2::gateChunk(n);
+    const uint32_t gateChunk = jgs2::gateChunk(n, sc.dynamic);
     for (uint32_t b0 = 0; b0 < std::max(n, 1u); b0 += gateChunk)
       gateTable.push_back({i, b0, std::min(n, b0 + gateChunk), static_cast<uint32_t>(gateTable.size())});
     r.gateBlocks = static_cast<uint32_t>(gateTable.size()) - r.gateBase;
@@ -2107,15 +2109,16 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
       STEP(upload(sp, &ks, contactScene.data(), nK));
       STEP(upload(sp, &kr, contactRange.data(), nV));
       STEP(upload(sp, &kd, contactIds.data(), contactIds.size()));
-      // Empty contact caches (distance -1), zero lagged records, neutral
-      // scratch (packIpcContactBuffer, ipc-contact-layout.ts:290-340).
-      std::vector<float4> state(7ull * nK, make_float4(0.f, 0.f, 0.f, 0.f));
+      // Empty contact caches (distance -1), zero lagged records
+      // (packIpcContactBuffer, ipc-contact-layout.ts:290-340).
+      std::vector<float4> state(6ull * nK, make_float4(0.f, 0.f, 0.f, 0.f));
       for (size_t c = 0; c < nK; ++c) {
-        state[7 * c + 0] = make_float4(0.f, 0.f, 0.f, -1.f);
-        state[7 * c + 2] = make_float4(0.f, 0.f, 0.f, -1.f);
-        state[7 * c + 6] = make_float4(1.f, 0.f, 0.f, 0.f);
+        state[6 * c + 0] = make_float4(0.f, 0.f, 0.f, -1.f);
+        state[6 * c + 2] = make_float4(0.f, 0.f, 0.f, -1.f);
       }
       STEP(upload(sp, &b.contactState, state.data(), state.size()));
+      STEP(deviceAlloc(sp, &b.contactNear, nK));
+      STEP(deviceAlloc(sp, &b.contactTargetNear, nK));
       STEP(deviceAlloc(sp, &b.activeCount, nV));
       STEP(deviceAlloc(sp, &b.activeIds, contactIds.size()));
       STEP(deviceAlloc(sp, &b.contactFlag, nK));
@@ -2166,7 +2169,7 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
       for (int l = 0; l < 2; ++l) {
         STEP(deviceAlloc(sp, &sp->dynIdx[l], cap));
         STEP(deviceAlloc(sp, &sp->dynScene[l], cap));
-        STEP(deviceAlloc(sp, &sp->dynState[l], 7 * cap));
+        STEP(deviceAlloc(sp, &sp->dynState[l], 6 * cap));
         STEP(deviceAlloc(sp, &sp->dynFlag[l], cap));
         STEP(deviceAlloc(sp, &sp->dynCols[l], cap));
         STEP(deviceAlloc(sp, &sp->dynRowOff[l], bpR + 1));
@@ -2177,6 +2180,11 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
       STEP(deviceAlloc(sp, &b.bpHist, 256 * ((4 * cap + 4095) / 4096) + 256));
       STEP(deviceAlloc(sp, &b.bpPinnedMove, nV));
       STEP(deviceAlloc(sp, &b.bpPrev, cap));
+      STEP(deviceAlloc(sp, &b.contactMove, nV));
+      STEP(deviceAlloc(sp, &b.bpRowHits, bpR * jgs2::kBpRowHits));
+      STEP(deviceAlloc(sp, &b.bpRowKept, bpR));
+      STEP(deviceAlloc(sp, &b.contactNear, cap));
+      STEP(deviceAlloc(sp, &b.contactTargetNear, cap));
       STEP(deviceAlloc(sp, &b.bpSpan, S));
       STEP(deviceAlloc(sp, &b.bpStatus, 4));
       CUDA_TRY(sp, cudaMemsetAsync(b.bpStatus, 0, sizeof(uint32_t) * 4, sp->stream));
@@ -3355,18 +3363,20 @@ uint64_t jgs2_estimate_device_bytes(const jgs2_input* in) {
   // 16-byte incidence range per vertex.
   const uint64_t C = in->cloth ? in->cloth->triangle_count : 0, H = in->cloth ? in->cloth->hinge_count : 0;
   const uint64_t cloth = (C + H) ? V * 16 + C * (32 + 12) + H * (32 + 16) : 0;
-  // IPC: per candidate its indices, scene, 7 float4 of state and four
+  // IPC: per candidate its indices, scene, 6 float4 of state, its two
+  // distances and four
   // incidence and four active entries; per vertex a range and an active count.
   const uint64_t KC = uint64_t(in->contact_vertex_triangle_count) + in->contact_edge_edge_count;
   uint64_t contact = KC ? KC * (16 + 4 + 112 + 32) + V * 12 : 0;
   if (const jgs2_contact_surface* cs = in->contact_surface) {
     // Broad phase: two lists of capacity candidates (indices, scene, state,
     // flag, column) and the sort's four entry buffers; surface data, boxes
-    // and rows per triangle and edge (at most three edges per triangle).
+    // and rows per triangle and edge (at most three edges per triangle), and
+    // each row's kept hit chunks.
     const uint64_t E = 3ull * cs->triangle_count;
     const uint64_t cap = cs->candidate_capacity ? cs->candidate_capacity : 65536 + 16 * (V + E);
     contact = 2 * cap * (16 + 4 + 112 + 4 + 4) + 4 * cap * 16 + cs->triangle_count * (16 + 32) + E * (8 + 32 + 32) +
-              V * (8 + 16 + 8 + 8 + 4 + 16) + (4 * cap / 4096 + 1) * 1024;
+              V * (8 + 16 + 8 + 8 + 4 + 16) + (4 * cap / 4096 + 1) * 1024 + (V + E) * (8 * 32 + 4);
   }
   return V * (16 * 20 + 12) + V * K * (32 + 144) + T * (64 + 16 + 1) + cloth + contact + (1u << 16);
 }
