@@ -47,6 +47,24 @@ def test_same_bits_in_both_forms(cells, filler):
     np.testing.assert_array_equal(a["history"], b["history"])
 
 
+# Cloth elements are added by the same lanes, in engines of up to 40 000
+# vertices: sheets of 33 and 1 164 vertices (with their collider's 8).
+@pytest.mark.parametrize("cells", [4, 33])
+def test_cloth_gives_the_same_bits_in_both_forms(cells):
+    inp = scenes.cloth_sheet(cells=cells)
+    settings = dict(scenes.CLOTH_SETTINGS)
+    alone = solver.JGS2GpuSolver.create(inp, settings)
+    both = solver.JGS2Batch.create([inp, _bar((34, 34, 34))], [settings, dict(SETTINGS, timestep=1 / 60)])
+    for _ in range(3):
+        alone.stepExactIterations(4)
+        both.stepFrames(1, 4)
+    np.testing.assert_array_equal(alone.readPositions(), both.readPositions(0))
+    np.testing.assert_array_equal(alone.readVelocities(), both.readVelocities(0))
+    a, b = alone.readGlobalizationDiagnostics(), both.readGlobalizationDiagnostics(0)
+    np.testing.assert_array_equal(a["local"], b["local"])
+    np.testing.assert_array_equal(a["history"], b["history"])
+
+
 @pytest.mark.parametrize("cells", [(7, 1, 1), (16, 3, 15), (20, 20, 20)])
 def test_frame_against_the_oracle(cells):
     inp = _bar(cells)

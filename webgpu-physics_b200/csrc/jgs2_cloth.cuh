@@ -93,10 +93,9 @@ __device__ __forceinline__ float3 clothMembraneGradient(const ClothTri& t, const
 }
 
 // Exact diagonal Hessian block of the membrane at the vertex in `slot`.
-__device__ __forceinline__ void clothMembraneHessian(S3& h, const ClothTri& t, const Membrane& e, uint32_t slot,
-                                                     const ClothMaterial& m) {
+__device__ __forceinline__ S3 clothMembraneBlock(const ClothTri& t, const Membrane& e, uint32_t slot,
+                                                 const ClothMaterial& m) {
   const float2 g = clothShapeGradient(t.inv, slot);
-  const float aw = t.area * m.thickness;
   const float gsg = g.x * g.x * e.s0 + 2.0f * g.x * g.y * e.s1 + g.y * g.y * e.s2;
   const float gg = g.x * g.x + g.y * g.y;
   const float3 u = e.f0 * g.x + e.f1 * g.y;
@@ -105,7 +104,11 @@ __device__ __forceinline__ void clothMembraneHessian(S3& h, const ClothTri& t, c
   saddOuter(blk, m.mu + m.lambda, u);
   saddOuter(blk, m.mu * gg, e.f0);
   saddOuter(blk, m.mu * gg, e.f1);
-  saddScaled(h, aw, blk);
+  return blk;
+}
+__device__ __forceinline__ void clothMembraneHessian(S3& h, const ClothTri& t, const Membrane& e, uint32_t slot,
+                                                     const ClothMaterial& m) {
+  saddScaled(h, t.area * m.thickness, clothMembraneBlock(t, e, slot, m));
 }
 
 // Signed relative area stretch |n| / 2A of a triangle (jgs2-shader.ts:2067-2116).
@@ -246,6 +249,45 @@ __device__ __forceinline__ void clothLocalSystem(const float4* __restrict__ tris
     gadd(grad, (ws * clothWrappedAngle(angle, rest.x)) * ag);
     if (kHessian) saddOuter(hess, ws, ag);
   }
+}
+
+// One cloth element's contribution at its vertex `slot`, as a row of factors:
+// the gradient (3) and six pairs whose products the Hessian sums take in one
+// fused step each, as clothLocalSystem's do.
+constexpr int kClothRow = 15;  // gradient 3, first factors 6, second factors 6
+__device__ __forceinline__ void clothTriangleRow(const float4* __restrict__ tris, uint32_t entry,
+                                                 const float4* __restrict__ x, const ClothMaterial& m, float* row) {
+  const uint32_t slot = entry & 3u;
+  const ClothTri t = loadClothTri(tris, entry >> 2);
+  const Membrane e = clothMembrane(t, xyz(x[t.i0]), xyz(x[t.i1]), xyz(x[t.i2]), m);
+  const float3 g = clothMembraneGradient(t, e, slot, m);
+  const S3 blk = clothMembraneBlock(t, e, slot, m);
+  const float aw = t.area * m.thickness;
+  row[0] = g.x; row[1] = g.y; row[2] = g.z;
+#pragma unroll
+  for (int i = 0; i < 6; ++i) row[3 + i] = aw;
+  row[9] = blk.xx; row[10] = blk.yy; row[11] = blk.zz; row[12] = blk.xy; row[13] = blk.xz; row[14] = blk.yz;
+}
+__device__ __forceinline__ void clothHingeRow(const float4* __restrict__ hinges, uint32_t entry,
+                                              const float4* __restrict__ x, const ClothMaterial& m, float* row) {
+  const uint32_t slot = entry & 3u, h = entry >> 2;
+  const uint4 q = hingeIndices(hinges, h);
+  const DihedralFrame f = clothDihedralFrame(xyz(x[q.x]), xyz(x[q.y]), xyz(x[q.z]), xyz(x[q.w]));
+  const float angle = f.valid ? atan2f(f.sine, f.cosine) : 0.0f;
+  const float3 ag = f.valid ? clothDihedralGradient(f, slot) : f3(0, 0, 0);
+#pragma unroll
+  for (int i = 0; i < kClothRow; ++i) row[i] = 0.0f;
+  if (!f.valid || !finiteS(angle) || !finiteV(ag)) {
+    row[0] = row[1] = row[2] = kF32Max;
+    return;
+  }
+  const float4 rest = __ldg(&hinges[2ull * h + 1]);
+  const float ws = m.bending * rest.y;
+  const float3 g = (ws * clothWrappedAngle(angle, rest.x)) * ag;
+  const float3 w = ws * ag;
+  row[0] = g.x; row[1] = g.y; row[2] = g.z;
+  row[3] = w.x; row[4] = w.y; row[5] = w.z; row[6] = w.x; row[7] = w.x; row[8] = w.y;
+  row[9] = ag.x; row[10] = ag.y; row[11] = ag.z; row[12] = ag.y; row[13] = ag.z; row[14] = ag.z;
 }
 
 }  // namespace jgs2

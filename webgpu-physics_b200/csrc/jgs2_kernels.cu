@@ -480,7 +480,9 @@ struct IncidentShared {
 enum IncidentPart { kFramePart, kSystemPart };
 template <IncidentPart kPart>
 __device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4* __restrict__ x, const uint4& info,
-                                                  float* rows, uint32_t lane, unsigned mask, float* out) {
+                                                  float* rows, uint32_t lane, unsigned mask, float* out,
+                                                 uint4 cloth = make_uint4(0u, 0u, 0u, 0u),
+                                                 const ClothMaterial& material = ClothMaterial{}) {
   float s[3] = {0.0f, 0.0f, 0.0f}, c = 0.0f;
   for (uint32_t a0 = 0; a0 < info.y; a0 += kIncidentLanes) {
     const uint32_t n = min(info.y - a0, static_cast<uint32_t>(kIncidentLanes));
@@ -529,6 +531,37 @@ __device__ __forceinline__ void incidentSumsLanes(const Buffers& b, const float4
     }
     __syncwarp(mask);
   }
+  if constexpr (kPart == kSystemPart) {
+    // The vertex's cloth triangles, then its hinges, a lane each likewise.
+    for (uint32_t a0 = 0; a0 < cloth.y + cloth.w;) {
+      const bool triangles = a0 < cloth.y;
+      const uint32_t end = triangles ? cloth.y : cloth.y + cloth.w;
+      const uint32_t n = min(end - a0, static_cast<uint32_t>(kIncidentLanes));
+      if (lane < n) {
+        float row[kClothRow];
+        if (triangles)
+          clothTriangleRow(b.clothTris, __ldg(&b.clothIncidence[cloth.x + a0 + lane]), x, material, row);
+        else
+          clothHingeRow(b.clothHinges, __ldg(&b.clothIncidence[cloth.z + a0 - cloth.y + lane]), x, material, row);
+#pragma unroll
+        for (int i = 0; i < kClothRow; ++i) rows[lane * kIncidentRow + i] = row[i];
+      }
+      __syncwarp(mask);
+      for (uint32_t j = 0; j < n; ++j) {
+        const float* q = rows + j * kIncidentRow;
+        if (lane < 3) {
+          float e;
+          s[0] = twoSum(s[0], q[lane], &e);
+          c = __fadd_rn(c, e);
+        } else {
+          s[0] = __fmaf_rn(q[lane], q[6 + lane], s[0]);
+        }
+        if (lane == 0) s[1] = __fmaf_rn(q[8], q[14], s[1]);
+      }
+      __syncwarp(mask);
+      a0 += n;
+    }
+  }
   out[lane] = s[0];
   out[8 + lane] = s[1];
   if (lane < 3) {
@@ -547,14 +580,17 @@ __device__ __forceinline__ IncidentSums loadIncidentSums(const float* q) {
 }
 // The sums of an entry's (at most 32) vertices, eight lanes per vertex, left
 // in shared memory (ends with a block barrier).
-__device__ __forceinline__ void incidentBlockSums(const Buffers& b, const float4* __restrict__ x, const RedBlock& rb,
-                                                  const SceneRange& sr, bool pinnedToo, IncidentShared& sh) {
+__device__ __forceinline__ void incidentBlockSums(const Buffers& b, const DevParams& p, const float4* __restrict__ x,
+                                                  const RedBlock& rb, const SceneRange& sr, bool pinnedToo,
+                                                  IncidentShared& sh) {
   const uint32_t group = threadIdx.x / kIncidentLanes, k = rb.begin + group;
   if (k < rb.end) {
     const uint4 info = b.vinfo[sr.vOff + k];
     if (pinnedToo || !isPinned(info))
       incidentSumsLanes<kSystemPart>(b, x, info, reinterpret_cast<float*>(sh.rows4) + group * kIncidentGroup,
-                              threadIdx.x % kIncidentLanes, 0xffu << (threadIdx.x & 24u), sh.sums[group]);
+                                     threadIdx.x % kIncidentLanes, 0xffu << (threadIdx.x & 24u), sh.sums[group],
+                                     p.cloth && !isPinned(info) ? b.clothRange[sr.vOff + k] : make_uint4(0u, 0u, 0u, 0u),
+                                     clothMaterial(p));
   }
   __syncthreads();
 }
@@ -565,8 +601,8 @@ __device__ __forceinline__ void incidentBlockSums(const Buffers& b, const float4
 // Hessian blocks plus the membrane and bending terms of the vertex's cloth.
 __device__ __forceinline__ void storeFrameAndIncident(const Buffers& b, const DevParams& p,
                                                       const float4* __restrict__ x, uint32_t v, const uint4& info,
-                                                      IncidentSums& o) {
-  if (p.cloth)
+                                                      IncidentSums& o, bool clothToo) {
+  if (p.cloth && clothToo)
     clothLocalSystem<true>(b.clothTris, b.clothHinges, b.clothIncidence, b.clothRange[v], x, clothMaterial(p), 0u, 1u,
                            o.grad, o.hess);
   const M3 favg = o.total > 0.0f ? (1.0f / o.total) * o.avg : midentity();
@@ -3948,7 +3984,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) prologueKernel(Bu
   if constexpr (kWide) {
     __shared__ IncidentShared shared;
     sh = &shared;
-    if (p.globalization) incidentBlockSums(b, b.pos[0], rb, sr, true, shared);
+    if (p.globalization) incidentBlockSums(b, p, b.pos[0], rb, sr, true, shared);
     if (threadIdx.x >= 32) return;
   }
   for (uint32_t k = rb.begin + lane; k < rb.end; k += 32) {
@@ -3981,7 +4017,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock) prologueKernel(Bu
       const M3 favg = sums.total > 0.0f ? (1.0f / sums.total) * sums.avg : midentity();
       storeFrame(b.vertexPack, i, info.y == 0u ? midentity() : polarRotation(favg, p.rotationEpsilon), xyz(o));
     } else {
-      storeFrameAndIncident(b, p, b.pos[0], i, info, sums);
+      storeFrameAndIncident(b, p, b.pos[0], i, info, sums, !kWide);
     }
     const float e = implicitEnergy(p, b, i, xyz(o), info);
     if (finiteS(e)) { acc.e0 += e; acc.e1 += e; }
@@ -4158,7 +4194,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock, kWide ? 2 : JGS2_
   if constexpr (kWide) {
     __shared__ IncidentShared shared;
     sh = &shared;
-    incidentBlockSums(b, acc, rb, sr, nextRotations != 0, shared);
+    incidentBlockSums(b, p, acc, rb, sr, nextRotations != 0, shared);
     if (threadIdx.x >= 32) return;
   }
   for (uint32_t k = rb.begin + lane; k < rb.end; k += 32) {
@@ -4184,7 +4220,7 @@ __global__ void __launch_bounds__(kWide ? kWideBlock : kBlock, kWide ? 2 : JGS2_
       comps[0] = (b.restMass[v].w * p.invDt2) * (x - xyz(b.predicted[v]));
       Comp3& material = sums.grad;
       S3& hess = sums.hess;
-      if (p.cloth) {
+      if (!kWide && p.cloth) {
         const uint4 cr = b.clothRange[v];
         if (nextRotations)
           clothLocalSystem<true>(b.clothTris, b.clothHinges, b.clothIncidence, cr, acc, clothMaterial(p), 0u, 1u,
@@ -4654,10 +4690,12 @@ uint32_t smCount() {
 // the timing itself), eight lanes against one thread: 525 vertices 17 / 26 us,
 // 2 688 vertices 19 / 27, 13 392 vertices 29 / 31, 27 360 vertices 41 / 35,
 // 68 921 vertices 98 / 57: past about ten thousand vertices the threads hide
-// each other's gathers.  Cloth adds its triangles and hinges one thread per
-// vertex whichever way the tets are summed, so it keeps that form.
+// each other's gathers.  A cloth vertex has some 18 elements of several
+// hundred operations, so there the lanes pay longer: sheets of 1 164 vertices
+// 21 / 41 us, 16 392 vertices 35 / 41.
 constexpr uint32_t kWideVertices = 8192;
-bool wideIncident(const Buffers& b) { return b.vertexTotal <= kWideVertices && !b.clothRange; }
+constexpr uint32_t kWideClothVertices = 40000;
+bool wideIncident(const Buffers& b) { return b.vertexTotal <= (b.clothRange ? kWideClothVertices : kWideVertices); }
 
 int launchPrologue(const Buffers& b, const DevParams* p, cudaStream_t s) {
   if (wideIncident(b)) prologueKernel<true><<<b.convBlocks, kWideBlock, 0, s>>>(b, p);
