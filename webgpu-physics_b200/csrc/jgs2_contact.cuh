@@ -4,11 +4,10 @@
 // the Lipschitz safe-step cap (src/simulation/gpu/ipc-contact-wgsl.ts:19-472
 // and the contact helpers of src/simulation/gpu/jgs2-shader.ts:233-874).
 //
-// Candidate state (7 float4 per candidate): source contact (normal,
+// Candidate state (6 float4 per candidate): source contact (normal,
 // distance; distance -1 when invalid) and its closest-feature weights, the
 // same for the target pose, the lagged normal force (normal, magnitude) and
-// its weights, and a scratch record.  Contact weights satisfy
-// sum_i w_i x_i = point_a - point_b.
+// its weights.  Contact weights satisfy sum_i w_i x_i = point_a - point_b.
 #pragma once
 
 #include "jgs2_device.cuh"

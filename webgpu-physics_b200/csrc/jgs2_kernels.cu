@@ -16,9 +16,9 @@
 // adds a copy and, per colour, a frame pass over the vertices that colour
 // reads plus an in-place solve over the colour's vertices.
 //
-// Grid-wide reductions finish in the last block to arrive (a ticket counter);
-// sums are combined in block order so results are deterministic.  No kernel
-// waits on another block.
+// Grid-wide reductions finish in the last block or warp to arrive (a ticket
+// counter); sums are combined in a fixed order so results are deterministic.
+// No kernel waits on another block.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -4735,11 +4735,10 @@ void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4
   uint32_t groups = kG;
   while (groups > 1 && itemSharedBytes(groups, K, !kJacobi, trials) > limit) --groups;
   groups = std::max(1u, groups >> shift);
-  static int attr = 0;
-  if (attr == 0) {
-    attr = static_cast<int>(limit);
-    cudaFuncSetAttribute(solveItemsKernel<kG, kThreads, kJacobi, kMin>, cudaFuncAttributeMaxDynamicSharedMemorySize, attr);
-  }
+  // The limit is a property of the device's copy of the kernel, so it is set at
+  // every launch (once per captured frame): engines may be on several devices.
+  cudaFuncSetAttribute(solveItemsKernel<kG, kThreads, kJacobi, kMin>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       static_cast<int>(limit));
   solveItemsKernel<kG, kThreads, kJacobi, kMin>
       <<<(count + groups - 1) / groups, kThreads, itemSharedBytes(groups, K, !kJacobi, trials), s>>>(
           b, p, src, tgt, list, count, K, groups);

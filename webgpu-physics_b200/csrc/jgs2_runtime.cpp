@@ -3354,8 +3354,8 @@ jgs2_status jgs2_batch_set_scene_active(jgs2_batch* s, uint32_t scene, uint32_t 
 uint64_t jgs2_estimate_device_bytes(const jgs2_input* in) {
   if (!in) return 0;
   const uint64_t V = in->vertex_count, T = in->tet_count, K = in->cubature_k;
-  // Per vertex: two position buffers, predicted, velocity, old, frame (3),
-  // local records (4), incident system (3), rest/mass, info, force, target
+  // Per vertex: two position buffers, predicted, velocity, old, the pack of
+  // frame, position and target (4), local records (4), incident system (3), rest/mass, info, force, target
   // (16 bytes each), final update, colour, scene id; per record a 32-byte
   // header and 144 bytes of basis; per tet a 64-byte record, four adjacency
   // entries and a share of the reduction partials; per cloth triangle and
@@ -3364,8 +3364,8 @@ uint64_t jgs2_estimate_device_bytes(const jgs2_input* in) {
   const uint64_t C = in->cloth ? in->cloth->triangle_count : 0, H = in->cloth ? in->cloth->hinge_count : 0;
   const uint64_t cloth = (C + H) ? V * 16 + C * (32 + 12) + H * (32 + 16) : 0;
   // IPC: per candidate its indices, scene, 6 float4 of state, its two
-  // distances and four
-  // incidence and four active entries; per vertex a range and an active count.
+  // distances, four incidence and four active entries; per vertex a range and
+  // an active count.
   const uint64_t KC = uint64_t(in->contact_vertex_triangle_count) + in->contact_edge_edge_count;
   uint64_t contact = KC ? KC * (16 + 4 + 112 + 32) + V * 12 : 0;
   if (const jgs2_contact_surface* cs = in->contact_surface) {
