@@ -2906,8 +2906,11 @@ __global__ void __launch_bounds__(kBlock, JGS2_SOLVE_MIN_BLOCKS) solveKernel(Buf
 // phases.  solveChunk's chain is two passes of four lanes over six records,
 // six passes over 24 incident tets per trial and up to 13 trials; here a
 // record or tet is one pass and, at eight vertices a block, a thread keeps its
-// incident tet's deformation gradient over the trials and four backtracked
-// trials are evaluated at a time.  Measured per launch (events; four lanes,
+// incident tet's deformation gradient over the trials and six backtracked
+// trials are evaluated at a time: a vertex that goes through all thirteen takes
+// three rounds, and six is what four summing lanes each leave room for (sweeps
+// of a colour-locked 525-vertex bar 4.99 ms two at a time, 4.36 four, 4.23
+// six; of a 27 360-vertex block 5.48, 4.98, 4.87).  Measured per launch (events; four lanes,
 // then items): 525 vertices 27.0 / 18.9 us, 2 688 vertices 35 / 27, 13 392
 // vertices 44.6 / 39.4; one colour of the 525-vertex bar, whose trials a
 // determinant bound often holds back, 72 / 33, of a 27 360-vertex block
@@ -2915,7 +2918,7 @@ __global__ void __launch_bounds__(kBlock, JGS2_SOLVE_MIN_BLOCKS) solveKernel(Buf
 // 1.72 ms, 1.79 by items, 68 921: 139 / 142 us): both run out of warps to hide
 // the gathers behind, and the block's barriers then cost more than the idle
 // lanes.
-constexpr uint32_t kItemTrials = 4;   // backtracked trials evaluated at a time
+constexpr uint32_t kItemTrials = 6;   // backtracked trials evaluated at a time
 constexpr uint32_t kItemTets = 24;    // incident tets of a vertex per round (the grid meshes' largest valence)
 constexpr uint32_t kBasisWords = 9;   // float4 per record: basis blocks, then dF (27), gQ (3), HQ (6)
 constexpr uint32_t kStateWords = 5;   // float4 per record: F, vol, lambda, mu, gs, w, I0, J0, slot; an odd stride
