@@ -872,6 +872,7 @@ struct Engine {
   uint32_t* dynFlag[2] = {nullptr, nullptr};
   uint32_t* dynCols[2] = {nullptr, nullptr};
   uint32_t* dynRowOff[2] = {nullptr, nullptr};
+  int lastList = 0;  // the list of the last iteration that listed candidates
   bool glob = true;
   std::vector<SceneHost> scenes;
   // Colour lists over all scenes: colour c holds every scene's colour-c vertices.
@@ -1092,6 +1093,18 @@ struct KernelProfiler {
   }
 };
 
+// The engine's buffers with the given one of its two candidate lists.
+Buffers withList(const Engine* s, int list) {
+  Buffers b = s->b;
+  b.contactIdx = s->dynIdx[list];
+  b.contactScene = s->dynScene[list];
+  b.contactState = s->dynState[list];
+  b.contactFlag = s->dynFlag[list];
+  b.bpCols = s->dynCols[list];
+  b.bpRowOff = s->dynRowOff[list];
+  return b;
+}
+
 // encodeFrame (src/simulation/gpu/jgs2-solver.ts:2207-2494) on the stream,
 // for every scene of the engine at once.  contact: some scene has IPC
 // contact this frame.
@@ -1152,12 +1165,7 @@ int encodeFrame(Engine* s, uint32_t iterations, uint32_t schedule, bool bodyCorr
     Buffers b = s->b;
     if (dynamic) {
       const int cur = static_cast<int>(it & 1u), prev = cur ^ 1;
-      b.contactIdx = s->dynIdx[cur];
-      b.contactScene = s->dynScene[cur];
-      b.contactState = s->dynState[cur];
-      b.contactFlag = s->dynFlag[cur];
-      b.bpCols = s->dynCols[cur];
-      b.bpRowOff = s->dynRowOff[cur];
+      b = withList(s, cur);
       b.bpPrevRowOff = s->dynRowOff[prev];
       b.bpPrevCols = s->dynCols[prev];
       b.bpPrevState = s->dynState[prev];
@@ -1357,6 +1365,7 @@ jgs2_status runFrames(Engine* s, const std::vector<jgs2_settings>& st, uint32_t 
     s->scenes[i].submittedIterations = iterations;
     if (s->glob) s->scenes[i].recordsAvailable = true;
   }
+  if (contact && iterations) s->lastList = static_cast<int>((iterations - 1) & 1u);
   return JGS2_OK;
 }
 
@@ -2194,13 +2203,8 @@ jgs2_status buildEngine(Engine* sp, const std::vector<PreparedScene>& prep, int 
       STEP(deviceAlloc(sp, &b.contactGrad, nV));
       CUDA_TRY(sp, cudaMemsetAsync(b.activeCount, 0, sizeof(uint32_t) * nV, sp->stream));
       CUDA_TRY(sp, cudaMemsetAsync(b.contactGrad, 0, sizeof(float4) * nV, sp->stream));
-      // The first list view; encodeFrame points each iteration at its own.
-      b.contactIdx = sp->dynIdx[0];
-      b.contactScene = sp->dynScene[0];
-      b.contactState = sp->dynState[0];
-      b.contactFlag = sp->dynFlag[0];
-      b.bpCols = sp->dynCols[0];
-      b.bpRowOff = sp->dynRowOff[0];
+      // The first list's view; encodeFrame points each iteration at its own.
+      b = withList(sp, 0);
       b.activeIds = b.bpVals[b.bpSortPasses & 1u];
     }
     STEP(upload(sp, &sp->dColorVertices, byColor.data(), byColor.size()));
@@ -2635,9 +2639,8 @@ jgs2_status jgs2_read_contact_candidates(jgs2_solver* s, uint32_t* out, uint64_t
   uint64_t n = sc.KC;
   uint64_t first = sc.kOff;
   if (s->dynamic) {
-    // The last iteration's list: the one its iteration count's parity picks.
-    const uint32_t it = sc.submittedIterations;
-    list = s->dynIdx[it ? static_cast<int>((it - 1) & 1u) : 0];
+    // The last iteration's list.
+    list = s->dynIdx[s->lastList];
     uint32_t total = 0;
     CUDA_TRY(s, cudaMemcpy(&total, s->b.bpStatus, sizeof(total), cudaMemcpyDeviceToHost));
     n = sc.submittedIterations ? total : 0u;
@@ -2910,7 +2913,9 @@ jgs2_status jgs2_evaluate_assembled_candidate(jgs2_solver* s, const float* sourc
   std::string err;
   if (!resolve(s->scenes[0].defaults, o, mask, &settings, &err)) return fail(s, JGS2_INVALID_ARGUMENT, err);
   s->hParams[0] = makeParams(s, 0, settings, false);
-  const Buffers& b = s->b;
+  // The contact terms are those of the last iteration's list: the distances,
+  // the spans and the promoted source caches are all of it.
+  const Buffers b = s->dynamic ? withList(s, s->lastList) : s->b;
   FrameState* fs = &b.frames[0];
   CUDA_TRY(s, cudaSetDevice(s->device));
   CUDA_TRY(s, cudaMemcpyAsync(s->dParams, &s->hParams[0], sizeof(DevParams), cudaMemcpyHostToDevice, s->stream));
