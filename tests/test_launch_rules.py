@@ -1,0 +1,58 @@
+"""Which kernel a launch takes and what it asks of the device, without a GPU:
+the host code of libjgs2.so launches against a pretended CUDA runtime
+(fake_cudart.cpp), which records kernels instead of running them and refuses
+what a device would refuse.
+"""
+import os
+import re
+import subprocess
+
+import pytest
+
+from jgs2_b200 import _ffi
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+CSRC = os.path.join(os.path.dirname(HERE), "webgpu-physics_b200", "csrc")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+@pytest.fixture(scope="module")
+def launch(tmp_path_factory):
+    """Runs script lines; per answered line (accepted, kernel with its template
+    arguments, device, grid, block, shared)."""
+    exe = str(tmp_path_factory.mktemp("fake") / "fake_cudart")
+    lib = os.path.abspath(_ffi.LIB_DIR)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(CUDA, "include"), "-I", CSRC,
+                    os.path.join(HERE, "fake_cudart.cpp"), "-o", exe, "-rdynamic", "-L", lib, "-ljgs2",
+                    f"-Wl,-rpath,{lib}", "-Wl,--allow-shlib-undefined"], check=True)
+
+    def run(*lines):
+        out = subprocess.run([exe], input="\n".join(lines) + "\n", capture_output=True, text=True, check=True).stdout
+        answers = []
+        for line in out.splitlines():
+            if line == "declined":
+                answers.append((False, "declined", ()))
+                continue
+            status, name, device, grid, block, shared = line.split()
+            kernel = re.search(r"\d(solveItemsKernel|solveKernel|coloredSweepKernel|convergenceKernel|prologueKernel)",
+                               name).group(1)
+            args = re.match(r"I((?:L[a-z]\d+E)+)E", name.split(kernel, 1)[1]).group(1)
+            kernel += "<" + ",".join(re.findall(r"L[a-z](\d+)E", args)) + ">"
+            answers.append((status == "ok", kernel, (int(device), int(grid), int(block), int(shared))))
+        return answers
+
+    return run
+
+
+# Twelve records a vertex take more shared memory than a kernel has without
+# asking: solid, cloth and contact solves, coloured lists, both sweeps, and the
+# item form, on the first device and on one after it.
+def test_every_device_may_use_its_shared_memory(launch):
+    calls = ["solve 50000 12 1 0 0 0 0", "solve 50000 12 1 1 0 0 0", "solve 200 12 0 0 100 1 0",
+             "solve 9000 12 0 0 0 1 0", "solve 2000 66 1 0 0 0 0", "sweep 12 0", "sweep 12 1"]
+    first = launch("device 0", *calls)
+    both = launch("device 0", *calls, "device 1", *calls)
+    assert all(ok for ok, _, _ in first) and len(first) == len(calls)
+    assert max(where[3] for _, _, where in first) > 48 * 1024
+    assert [(ok, kernel) for ok, kernel, _ in both] == 2 * [(ok, kernel) for ok, kernel, _ in first]
+    assert [where[0] for _, _, where in both] == [0] * len(calls) + [1] * len(calls)

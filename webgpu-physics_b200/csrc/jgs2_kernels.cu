@@ -4728,6 +4728,13 @@ int launchVertexPolar(const Buffers& b, const DevParams* p, const float4* src, c
   return 1;
 }
 
+// Lets `kernel` use `bytes` of dynamic shared memory on the current device.
+// The limit is a property of the device's copy of the kernel, so it is set at
+// every launch (once per captured frame): engines may be on several devices.
+void allowShared(const void* kernel, uint32_t bytes) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+}
+
 template <uint32_t kG, uint32_t kThreads, bool kJacobi, int kMin>
 void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
                  uint32_t count, uint32_t K, uint32_t shift, cudaStream_t s) {
@@ -4738,10 +4745,7 @@ void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4
   uint32_t groups = kG;
   while (groups > 1 && itemSharedBytes(groups, K, !kJacobi, trials) > limit) --groups;
   groups = std::max(1u, groups >> shift);
-  // The limit is a property of the device's copy of the kernel, so it is set at
-  // every launch (once per captured frame): engines may be on several devices.
-  cudaFuncSetAttribute(solveItemsKernel<kG, kThreads, kJacobi, kMin>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       static_cast<int>(limit));
+  allowShared(reinterpret_cast<const void*>(solveItemsKernel<kG, kThreads, kJacobi, kMin>), limit);
   solveItemsKernel<kG, kThreads, kJacobi, kMin>
       <<<(count + groups - 1) / groups, kThreads, itemSharedBytes(groups, K, !kJacobi, trials), s>>>(
           b, p, src, tgt, list, count, K, groups);
@@ -4768,6 +4772,15 @@ bool launchSolveItems(const Buffers& b, const DevParams* p, const float4* src, f
     else return false;
   }
   return true;
+}
+
+// solveKernel with its records cached in `shared` bytes.
+template <int W, bool kExt>
+void launchCached(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
+                  uint32_t count, uint32_t K, int ci, uint32_t groups, uint32_t blocks, uint32_t threads,
+                  size_t shared, cudaStream_t s) {
+  allowShared(reinterpret_cast<const void*>(solveKernel<W, kExt, true>), solveSharedBytes());
+  solveKernel<W, kExt, true><<<blocks, threads, shared, s>>>(b, p, src, tgt, list, count, K, ci, groups);
 }
 
 int launchSolve(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
@@ -4799,22 +4812,20 @@ int launchSolve(const Buffers& b, const DevParams* p, const float4* src, float4*
     const size_t wsmem = cache ? static_cast<size_t>(wg) * K * kSolveSlotBytes : 0;
     const uint32_t wb = std::max(1u, (count + wg - 1) / wg);
     if (cache)
-      solveKernel<32, true, true><<<wb, wg * 32, wsmem, s>>>(b, p, src, tgt, list, count, K, ci, wg);
+      launchCached<32, true>(b, p, src, tgt, list, count, K, ci, wg, wb, wg * 32, wsmem, s);
     else
       solveKernel<32, true, false><<<wb, wg * 32, 0, s>>>(b, p, src, tgt, list, count, K, ci, wg);
   } else if (b.clothRange || b.contactIdx) {
-    if (cache) solveKernel<kGroup, true, true><<<blocks, threads, smem, s>>>(b, p, src, tgt, list, count, K, ci, groups);
+    if (cache) launchCached<kGroup, true>(b, p, src, tgt, list, count, K, ci, groups, blocks, threads, smem, s);
     else solveKernel<kGroup, true, false><<<blocks, threads, 0, s>>>(b, p, src, tgt, list, count, K, ci, groups);
   } else if (cache && K > 0 && launchSolveItems(b, p, src, tgt, list, count, K, cachedIncident, shift, s)) {
   } else {
-    if (cache) solveKernel<kGroup, false, true><<<blocks, threads, smem, s>>>(b, p, src, tgt, list, count, K, ci, groups);
+    if (cache) launchCached<kGroup, false>(b, p, src, tgt, list, count, K, ci, groups, blocks, threads, smem, s);
     else solveKernel<kGroup, false, false><<<blocks, threads, 0, s>>>(b, p, src, tgt, list, count, K, ci, groups);
   }
   return 1;
 }
 
-// Dynamic shared memory a solve block may use (the device's opt-in limit less
-// the kernel's static shared memory); sets the kernels' attribute once.
 int launchColoredSweep(const Buffers& b, const DevParams* p, float4* x, const uint32_t* colorVertices,
                        const uint32_t* colorOffsets, const uint32_t* needVertices, const uint32_t* needOffsets,
                        uint32_t colorCount, uint32_t V, uint32_t K, uint32_t largestColor, uint32_t largestNeed,
@@ -4829,12 +4840,7 @@ int launchColoredSweep(const Buffers& b, const DevParams* p, float4* x, const ui
   const bool ext = b.clothRange || b.contactIdx;
   const void* fn = ext ? reinterpret_cast<const void*>(coloredSweepKernel<kGroup, true>)
                        : reinterpret_cast<const void*>(coloredSweepKernel<kGroup, false>);
-  static int attr = -1;
-  if (attr < 0) {
-    attr = static_cast<int>(solveSharedBytes());
-    cudaFuncSetAttribute(coloredSweepKernel<kGroup, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, attr);
-    cudaFuncSetAttribute(coloredSweepKernel<kGroup, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, attr);
-  }
+  allowShared(fn, solveSharedBytes());
   int device = 0, sms = 0, perSm = 0;
   cudaGetDevice(&device);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
@@ -4890,17 +4896,10 @@ cudaError_t takeBoundsViolation(uint32_t* site) {
 }
 
 uint32_t solveSharedBytes() {
-  static int optin = -1;
-  if (optin < 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 48 * 1024;
-    optin -= 1024;  // static shared memory of the kernel
-    cudaFuncSetAttribute(solveKernel<kGroup, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    cudaFuncSetAttribute(solveKernel<kGroup, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-    cudaFuncSetAttribute(solveKernel<32, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
-  }
-  return static_cast<uint32_t>(optin);
+  int dev = 0, optin = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) optin = 48 * 1024;
+  return static_cast<uint32_t>(optin - 1024);  // static shared memory of the kernel
 }
 
 bool solveCachesRecords(uint32_t K) { return static_cast<size_t>(K) * kSolveSlotBytes <= kSolveCacheBytesPerVertex; }

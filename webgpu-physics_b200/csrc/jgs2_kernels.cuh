@@ -311,7 +311,8 @@ uint32_t solveGroupsPerBlock(uint32_t K);
 // Whether the solve caches records of width K in shared memory (else it
 // recomputes them in the line search).
 bool solveCachesRecords(uint32_t K);
-// Dynamic shared memory available to one solve block.
+// Dynamic shared memory one solve block may use on the current device (its
+// opt-in limit less the kernel's static shared memory).
 uint32_t solveSharedBytes();
 constexpr size_t kGatePartialBytes = 32;
 constexpr size_t kConvPartialBytes = 80;
