@@ -56,3 +56,20 @@ def test_every_device_may_use_its_shared_memory(launch):
     assert max(where[3] for _, _, where in first) > 48 * 1024
     assert [(ok, kernel) for ok, kernel, _ in both] == 2 * [(ok, kernel) for ok, kernel, _ in first]
     assert [where[0] for _, _, where in both] == [0] * len(calls) + [1] * len(calls)
+
+
+def _forms(answers):
+    return [kernel for _, kernel, _ in answers]
+
+
+# The item form's size rules are in waves of the device's own blocks.
+@pytest.mark.parametrize("sms", [148, 100, 74])
+def test_item_forms_follow_the_device(launch, sms):
+    wave = 2 * sms
+    script = [f"sms {sms}"]
+    script += [f"solve {n} 6 1 0 0 0 0" for n in (1, 8 * wave, 8 * wave + 1, 16 * wave, 16 * wave + 1)]
+    script += [f"solve {n} 6 0 0 0 1 0" for n in (1, 24 * wave, 24 * wave + 1)]
+    assert _forms(launch(*script)) == [
+        "solveItemsKernel<8,192,1,2>", "solveItemsKernel<8,192,1,2>", "solveItemsKernel<16,192,1,2>",
+        "solveItemsKernel<16,192,1,2>", "solveItemsKernel<32,160,1,3>", "solveItemsKernel<8,192,0,2>",
+        "solveItemsKernel<8,192,0,2>", "solveKernel<4,0,1>"]

@@ -4678,13 +4678,11 @@ __global__ void __launch_bounds__(1024) oracleReduceKernel(OracleParams q, const
 
 inline uint32_t blocksFor(uint32_t n) { return (n + kBlock - 1) / kBlock; }
 
+// SMs of the current device.
 uint32_t smCount() {
-  static int sms = 0;
-  if (sms == 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-  }
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
   return static_cast<uint32_t>(sms);
 }
 
@@ -4758,17 +4756,17 @@ void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4
 // for three waves of blocks (3 650 vertices per colour: 60 us, 64 with sixteen,
 // 71 with four lanes); past that four lanes (10 300 per colour: 90 us, 105 with
 // sixteen, 117 with eight).
-constexpr uint32_t kItemBlocks = 296;  // two per SM
 constexpr uint32_t kItemLargest = 40000;
 bool launchSolveItems(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
                       uint32_t count, uint32_t K, bool jacobi, uint32_t shift, cudaStream_t s) {
+  const uint32_t wave = 2 * smCount();  // blocks, two per SM
   if (jacobi) {
-    if (count <= 8 * kItemBlocks) launchItems<8, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
-    else if (count <= 16 * kItemBlocks) launchItems<16, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
+    if (count <= 8 * wave) launchItems<8, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
+    else if (count <= 16 * wave) launchItems<16, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
     else if (count <= kItemLargest) launchItems<32, 160, true, 3>(b, p, src, tgt, list, count, K, shift, s);
     else return false;
   } else {
-    if (count <= 3 * 8 * kItemBlocks) launchItems<8, 192, false, 2>(b, p, src, tgt, list, count, K, shift, s);
+    if (count <= 3 * 8 * wave) launchItems<8, 192, false, 2>(b, p, src, tgt, list, count, K, shift, s);
     else return false;
   }
   return true;
