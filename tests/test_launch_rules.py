@@ -73,3 +73,12 @@ def test_item_forms_follow_the_device(launch, sms):
         "solveItemsKernel<8,192,1,2>", "solveItemsKernel<8,192,1,2>", "solveItemsKernel<16,192,1,2>",
         "solveItemsKernel<16,192,1,2>", "solveItemsKernel<32,160,1,3>", "solveItemsKernel<8,192,0,2>",
         "solveItemsKernel<8,192,0,2>", "solveKernel<4,0,1>"]
+
+
+# Eight lanes per vertex in the incident passes: solids up to 8 192 vertices,
+# engines with cloth up to 28 672, the lanes' break-even there.
+@pytest.mark.parametrize("kernel", ["convergence", "prologue"])
+def test_the_incident_passes_change_form_where_both_measure_alike(launch, kernel):
+    sizes = [(1, 0), (8192, 0), (8193, 0), (16392, 1), (28672, 1), (28673, 1), (32769, 1)]
+    got = _forms(launch(*[f"{kernel} {v} {cloth}" for v, cloth in sizes]))
+    assert got == [f"{kernel}Kernel<{wide}>" for wide in (1, 1, 0, 1, 1, 0, 0)]

@@ -4691,11 +4691,19 @@ uint32_t smCount() {
 // the timing itself), eight lanes against one thread: 525 vertices 17 / 26 us,
 // 2 688 vertices 19 / 27, 13 392 vertices 29 / 31, 27 360 vertices 41 / 35,
 // 68 921 vertices 98 / 57: past about ten thousand vertices the threads hide
-// each other's gathers.  A cloth vertex has some 18 elements of several
-// hundred operations, so there the lanes pay longer: sheets of 1 164 vertices
-// 21 / 41 us, 16 392 vertices 35 / 41.
+// each other's gathers.
+//   With cloth the lanes pay longer, and it is the engine's whole size that
+// decides, not its share of cloth: a cloth vertex has some 18 elements of
+// several hundred operations, and by one thread even a few of them set the
+// time of the launch (a 27 000-vertex solid alone 37 / 33 us, with a sheet of
+// 81 vertices 40 / 51).  Sheets of 16 392 vertices 35 / 46, 22 809 46 / 50,
+// 32 769 58 / 51; solids with sheets: 8 820 + 16 384 44 / 52, 19 683 + 10 201
+// 49 / 52, 8 820 + 22 801 55 / 52.  A frame also has one prologue, where the
+// lanes stop paying sooner (22 809-vertex sheet 64 / 56, 27 000 + 1 681 73 /
+// 54): with four iterations a frame both forms take the same time between
+// 28 000 and 31 000 vertices, whatever the mix.
 constexpr uint32_t kWideVertices = 8192;
-constexpr uint32_t kWideClothVertices = 40000;
+constexpr uint32_t kWideClothVertices = 28672;
 bool wideIncident(const Buffers& b) { return b.vertexTotal <= (b.clothRange ? kWideClothVertices : kWideVertices); }
 
 int launchPrologue(const Buffers& b, const DevParams* p, cudaStream_t s) {
