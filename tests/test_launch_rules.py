@@ -82,3 +82,19 @@ def test_the_incident_passes_change_form_where_both_measure_alike(launch, kernel
     sizes = [(1, 0), (8192, 0), (8193, 0), (16392, 1), (28672, 1), (28673, 1), (32769, 1)]
     got = _forms(launch(*[f"{kernel} {v} {cloth}" for v, cloth in sizes]))
     assert got == [f"{kernel}Kernel<{wide}>" for wide in (1, 1, 0, 1, 1, 0, 0)]
+
+
+# 32 vertices a block by item only where shared memory holds as many blocks as
+# of four lanes, or one wave of them takes every vertex: not at 8 and 9 records
+# past 9 472 vertices (148 SMs), nor at 12 to 14.
+@pytest.mark.parametrize("vertices", [4737, 9472, 9473, 40000])
+def test_wide_blocks_by_item_need_room(launch, vertices):
+    widths = [1, 4, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 24, 40, 68]
+    got = _forms(launch(*[f"solve {vertices} {k} 1 0 0 0 0" for k in widths]))
+    lanes = {12, 13, 14} | ({8, 9} if vertices > 9472 else set())
+    want = ["solveKernel<4,0,1>" if k in lanes else "solveItemsKernel<32,160,1,3>" for k in widths]
+    assert got == want
+    # The smaller forms take every width.
+    for n, form in ((2368, 8), (4736, 16)):
+        small = _forms(launch(*[f"solve {n} {k} 1 0 0 0 0" for k in widths]))
+        assert small == [f"solveItemsKernel<{form},192,1,2>"] * len(widths)

@@ -4763,15 +4763,40 @@ void launchItems(const Buffers& b, const DevParams* p, const float4* src, float4
 // eight, 37 with 32), then 32 on three blocks per SM.  Coloured lists: eight
 // for three waves of blocks (3 650 vertices per colour: 60 us, 64 with sixteen,
 // 71 with four lanes); past that four lanes (10 300 per colour: 90 us, 105 with
-// sixteen, 117 with eight).
+// sixteen, 117 with eight).  Those are six records a vertex; of other counts
+// (1 to 66) the forms of eight and sixteen, and the coloured lists, are the
+// faster ones throughout (525 vertices 24 records 21 / 46 us, 60 records
+// 29 / 96; 2 750 vertices 12 records 23 / 34, 24 records 43 / 46), and the form
+// of 32 where itemRoom says.
 constexpr uint32_t kItemLargest = 40000;
+
+// Whether an SM's shared memory holds as many blocks of 32 vertices by item (a
+// record takes 296 bytes there, 240 with four lanes) as of four lanes, of which
+// only three count, or one wave of blocks takes all vertices.  Measured per
+// launch, items / four lanes: 27 000 vertices 6 records 63 / 75 us, 8 records
+// 74 / 68, 9 records 85 / 90, 10 records 81 / 96, 12 records 152 / 112, 14
+// records 157 / 134, 16 records 181 / 187, 24 records 251 / 264, 60 records
+// 556 / 1 084; 39 304 vertices 8 records 119 / 101, 9 records 130 / 123, 10
+// records 135 / 155, 12 records 244 / 172, 16 records 280 / 283.  At 8 and 9 records two blocks by item stand against three
+// of four lanes, at 12 to 14 one against two; 8 820 vertices, which two blocks
+// per SM take in one wave, 8 records 29 / 33, 9 records 31 / 41.
+bool itemRoom(uint32_t count, uint32_t K) {
+  constexpr uint32_t kG = 32;
+  int dev = 0, perSm = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&perSm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) return true;
+  auto resident = [&](size_t bytes) { return std::max<size_t>(1, perSm / (bytes + 1024)); };  // 1 KB is the system's
+  const size_t items = resident(itemSharedBytes(kG, K, false, 1u) + sizeof(ItemShared<kG, 1u>));
+  const size_t lanes = std::min<size_t>(3, resident(size_t(kG) * K * kSolveSlotBytes + 1024));
+  return items >= lanes || count <= kG * items * smCount();
+}
 bool launchSolveItems(const Buffers& b, const DevParams* p, const float4* src, float4* tgt, const uint32_t* list,
                       uint32_t count, uint32_t K, bool jacobi, uint32_t shift, cudaStream_t s) {
   const uint32_t wave = 2 * smCount();  // blocks, two per SM
   if (jacobi) {
     if (count <= 8 * wave) launchItems<8, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
     else if (count <= 16 * wave) launchItems<16, 192, true, 2>(b, p, src, tgt, list, count, K, shift, s);
-    else if (count <= kItemLargest) launchItems<32, 160, true, 3>(b, p, src, tgt, list, count, K, shift, s);
+    else if (count <= kItemLargest && itemRoom(count, K)) launchItems<32, 160, true, 3>(b, p, src, tgt, list, count, K, shift, s);
     else return false;
   } else {
     if (count <= 3 * 8 * wave) launchItems<8, 192, false, 2>(b, p, src, tgt, list, count, K, shift, s);
