@@ -3242,8 +3242,14 @@ __global__ void __launch_bounds__(kItemThreads, kMinBlocks)
   const bool summing = sg < n && sh.solve[sg] != 0u;
   Comp3 gsum = czero();
   S3 hess = szero();
+  // A checked build may reject a tet that the sums go over: its terms are none.
+  constexpr bool kRejects = JGS2_BOUNDS_CHECKS != 0;
   auto incidentRow = [&](uint32_t i, const HeldTet& h) {
-    if (!h.ok) return;
+    if (!h.ok) {
+      if (kRejects)
+        for (uint32_t k = 0; k < kTetRowFloats; ++k) tetRows[i * kTetRowFloats + k] = 0.0f;
+      return;
+    }
     float3 f;
     S3 blk;
     fused::incident(h.F, h.g, h.vol, h.lambda, h.mu, &f, &blk);
@@ -3483,7 +3489,15 @@ __global__ void __launch_bounds__(kItemThreads, kMinBlocks)
         HeldTet h;
         if (kHold && a0 == 0) h = held;
         else loadHeld(g, a0 + i % kItemTets, h);
-        if (!h.ok) continue;
+        if (!h.ok) {
+          if (kRejects)
+            for (uint32_t j = 0; j < trials; ++j) {
+              float* t = tetTrial + j * tetStride + 3u * i;
+              t[0] = t[1] = 0.0f;
+              t[2] = kF32Max;
+            }
+          continue;
+        }
         for (uint32_t j = 0; j < trials; ++j) {
           float J = 0.0f;
           const float e = fused::energyDelta(h.F, f3(sh.td[j][g][0], sh.td[j][g][1], sh.td[j][g][2]), h.g, h.lambda,
