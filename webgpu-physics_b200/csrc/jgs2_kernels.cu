@@ -1550,7 +1550,6 @@ __global__ void __launch_bounds__(kBlock) contactPromoteKernel(Buffers b, const 
 // row keeps ascending candidate order, as the static rows do.
 
 constexpr uint32_t kBpChunk = 32;
-constexpr uint32_t kBpKept = kBpRowHits;
 constexpr uint32_t kBpClosedMax = 64;  // closed one-ring vertices a row keeps in shared memory
 constexpr float kBpInf = __builtin_huge_valf();
 
@@ -1777,7 +1776,7 @@ __global__ void JGS2_CONTACT_BOUNDS bpInitKernel(Buffers b, const DevParams* __r
 
 // One warp per row: the row's pairs in column order, counted (kWrite false,
 // into bpRowOff[row]) or placed at the row's offset with their previous
-// entry (kWrite true).  The count keeps a row's first kBpKept hit chunks with
+// entry (kWrite true).  The count keeps a row's first kBpRowHits hit chunks with
 // their masks, from which the write pass places the pairs without testing any
 // box; a row with more walks them again.  The columns are walked 32 superchunks (of 32 chunks
 // of 32 primitives) at a time, then 32 chunks, then 32 primitives, each
@@ -1862,8 +1861,8 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
     uint2 mine = make_uint2(0u, 0u);
     if constexpr (kWrite) {
       const uint32_t n = b.bpRowKept[r];
-      if (n <= kBpKept) {
-        if (lane < n) mine = b.bpRowHits[static_cast<size_t>(r) * kBpKept + lane];
+      if (n <= kBpRowHits) {
+        if (lane < n) mine = b.bpRowHits[static_cast<size_t>(r) * kBpRowHits + lane];
         for (uint32_t i = 0; i < n; ++i) place(__shfl_sync(0xffffffffu, mine.x, i), __shfl_sync(0xffffffffu, mine.y, i));
         return;
       }
@@ -1979,7 +1978,7 @@ __global__ void __launch_bounds__(kBlock) bpRowsKernel(Buffers b, const DevParam
       }
     }
     if constexpr (!kWrite) {
-      if (lane < kept) b.bpRowHits[static_cast<size_t>(r) * kBpKept + lane] = mine;
+      if (lane < kept) b.bpRowHits[static_cast<size_t>(r) * kBpRowHits + lane] = mine;
       if (lane == 0) b.bpRowKept[r] = kept;
     }
   }
@@ -3972,16 +3971,17 @@ __device__ __forceinline__ void accumulateHinge(GatePartial& acc, const float4* 
   if (finiteS(ec)) acc.e1 += ec; else acc.bits &= ~kCandidateEnergyValid;
 }
 
-// ---------------------------------------------------------------------------
-// Prologue: predict (jgs2-shader.ts:2660-2692), iteration-0 vertex frames and
-// the source feasibility preflight (candidateTetrahedron + reduceCandidate on
-// the accepted pose, jgs2-solver.ts:2240-2259).
-// Elements [x, y) of `n` that fall to a scene's convergence block.
+// Elements [x, y) of `n` that fall to a scene's reduction entry.
 __device__ __forceinline__ uint2 blockShare(uint32_t n, const RedBlock& rb, const SceneRange& sr) {
   const uint64_t i = rb.slot - sr.convBase;
   return make_uint2(static_cast<uint32_t>(n * i / sr.convBlocks), static_cast<uint32_t>(n * (i + 1) / sr.convBlocks));
 }
 
+// ---------------------------------------------------------------------------
+// Prologue: predict (jgs2-shader.ts:2660-2692), iteration-0 vertex frames and
+// the source feasibility preflight (candidateTetrahedron + reduceCandidate on
+// the accepted pose, jgs2-solver.ts:2240-2259).
+//
 // One warp per reduction entry: its vertices, and its share of the scene's
 // tets, cloth triangles and hinges, so every warp has the same mix of work.
 // kWide: a block per entry, whose eight warps first form the incident sums.
