@@ -862,7 +862,13 @@ __device__ __forceinline__ float corotatedRecord(const Buffers& b, const DevPara
     // belongs to the vertex, not to the record).
     const float3 away = position - xyz(pv);
     pg = pg - (own + f3(__fmul_rn(dWs, away.x), __fmul_rn(dWs, away.y), __fmul_rn(dWs, away.z)));
-    if (objActive) pg = pg - distributedObjective(p, b, v, position, info);
+    if (objActive) {
+      // The vertex's own share (it is not pinned) in one rounding, as the
+      // one-thread-per-vertex form, which knew that, was contracted.
+      const float3 og = objectiveGradient(p, b, v, position);
+      const float share = 1.0f / float(info.y > 1u ? info.y : 1u);
+      pg = f3(__fmaf_rn(-og.x, share, pg.x), __fmaf_rn(-og.y, share, pg.y), __fmaf_rn(-og.z, share, pg.z));
+    }
     ph = ph - (mm(mm(R, stiffnessBlock(k, ss, ss)), mtrans(R)) + dWs * midentity());
     if (p.objectiveFlags & 2u)
       ph = ph - (targetStiffness(p, b, v) / float(info.y > 1u ? info.y : 1u)) * midentity();
