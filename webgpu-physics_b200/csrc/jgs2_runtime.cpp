@@ -3369,18 +3369,19 @@ uint64_t jgs2_estimate_device_bytes(const jgs2_input* in) {
   const uint64_t C = in->cloth ? in->cloth->triangle_count : 0, H = in->cloth ? in->cloth->hinge_count : 0;
   const uint64_t cloth = (C + H) ? V * 16 + C * (32 + 12) + H * (32 + 16) : 0;
   // IPC: per candidate its indices, scene, 6 float4 of state, its two
-  // distances, four incidence and four active entries; per vertex a range and
-  // an active count.
+  // distances, flag, four incidence and four active entries; per vertex a
+  // range and an active count.
+  constexpr uint64_t state = 6 * 16, distances = 2 * 4;
   const uint64_t KC = uint64_t(in->contact_vertex_triangle_count) + in->contact_edge_edge_count;
-  uint64_t contact = KC ? KC * (16 + 4 + 112 + 32) + V * 12 : 0;
+  uint64_t contact = KC ? KC * (16 + 4 + state + distances + 4 + 32) + V * 12 : 0;
   if (const jgs2_contact_surface* cs = in->contact_surface) {
     // Broad phase: two lists of capacity candidates (indices, scene, state,
-    // flag, column) and the sort's four entry buffers; surface data, boxes
-    // and rows per triangle and edge (at most three edges per triangle), and
-    // each row's kept hit chunks.
+    // flag, column), a candidate's distances and previous entry, and the sort's
+    // four entry buffers; surface data, boxes and rows per triangle and edge (at
+    // most three edges per triangle), and each row's kept hit chunks.
     const uint64_t E = 3ull * cs->triangle_count;
     const uint64_t cap = cs->candidate_capacity ? cs->candidate_capacity : 65536 + 16 * (V + E);
-    contact = 2 * cap * (16 + 4 + 112 + 4 + 4) + 4 * cap * 16 + cs->triangle_count * (16 + 32) + E * (8 + 32 + 32) +
+    contact = 2 * cap * (16 + 4 + state + 4 + 4) + cap * (distances + 4) + 4 * cap * 16 + cs->triangle_count * (16 + 32) + E * (8 + 32 + 32) +
               V * (8 + 16 + 8 + 8 + 4 + 16) + (4 * cap / 4096 + 1) * 1024 + (V + E) * (8 * 32 + 4);
   }
   return V * (16 * 20 + 12) + V * K * (32 + 144) + T * (64 + 16 + 1) + cloth + contact + (1u << 16);
